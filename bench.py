@@ -57,8 +57,7 @@ FALLBACK_HBM_GBS = 6650.0
 # 8 B each), isothermal / with energy equation.
 STAGE_BYTES = {
     "cfl_forces": (32, 40), "potential": (8, 8), "soundspeed": (0, 24),
-    "substep1": (64, 64), "viscous_terms": (56, 56), "viscous_update": (64, 64),
-    "substep2": (40, 56), "substep3": (0, 80),
+    "substep1": (64, 64), "source_terms": (40, 56), "substep3": (0, 40),
     "transport_radial": (64, 80), "transport_azimuthal": (80, 96),
     "transport_vr_boundary": (40, 40), "transport_ring_means": (8, 8),
 }

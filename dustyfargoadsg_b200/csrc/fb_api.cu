@@ -11,14 +11,11 @@
 
 #define FB_PROFILE_POINTS 64
 enum {
-  ST_CFL, ST_SUB0, ST_CONTROL, ST_SOUND, ST_POT, ST_SUB1, ST_SG, ST_SGCOLS, ST_SGINV, ST_SGUPD,
-  ST_VTERMS, ST_VUPDATE,
-  ST_SUB2, ST_EVTERMS, ST_SUB3, ST_TRAD, ST_TAZI, ST_TVR, ST_DAMP, ST_DUST, ST_TVMED, FB_NSTAGE
+  ST_CFL, ST_SUB0, ST_SOUND, ST_POT, ST_SUB1, ST_SG, ST_SGCOLS, ST_SGINV, ST_SRC, ST_SUB3, ST_TRAD, ST_TAZI, ST_TVR, ST_DAMP, ST_DUST, ST_TVMED, FB_NSTAGE
 };
 static const char *stage_names[FB_NSTAGE] = {
-  "cfl_forces", "substep0", "controller", "soundspeed", "potential", "substep1", "sg_rows_fwd",
-  "sg_cols", "sg_rows_inv", "sg_update",
-  "viscous_terms", "viscous_update", "substep2", "energy_viscous_terms", "substep3",
+  "cfl_forces", "substep0", "soundspeed", "potential", "substep1", "sg_rows_fwd", "sg_cols", "sg_rows_inv",
+  "source_terms", "substep3",
   "transport_radial", "transport_azimuthal", "transport_vr_boundary", "damping", "dust_particles",
   "transport_ring_means"};
 
@@ -362,6 +359,12 @@ extern "C" int fb_create(const fb_params *p, const double *radii, fb_ctx **out)
   k.vthetamed = dalloc(ctx, nr);
   k.vradmed = dalloc(ctx, nr);
   k.betatab = dtable(ctx, beta.data(), nr);
+  {
+    std::vector<double> st((size_t)nr * FB_SRC_TAB);
+    fb_source_table(&g, invdxth.data(), p15.data(), cs_ring.data(), st.data());
+    k.src_tab = dtable(ctx, st.data(), st.size());
+    if (!k.src_tab) { fb_destroy(ctx); return FB_ERR_NOMEM; }
+  }
   k.damp_lam = dtable(ctx, dlam.data(), nr);
   k.damp_tau = dtable(ctx, dtau.data(), nr);
   {
@@ -378,7 +381,13 @@ extern "C" int fb_create(const fb_params *p, const double *radii, fb_ctx **out)
   k.vh_l2 = log(g.rmed[1] / g.rmed[2]);
   k.ringmin = dalloc(ctx, nr);
   k.vmoy = dalloc(ctx, nr);
-  k.vt_part = dalloc(ctx, (size_t)nr * ((ns + 31) / 32));  // CTAs of >= 32 azimuths
+  k.vt_part = dalloc(ctx, (size_t)nr * fb_source_tiles(ns));
+  if (!k.vt_part) { fb_destroy(ctx); return FB_ERR_NOMEM; }
+  // scratch free during the substep (the stress fields serve the viscous stage
+  // on its own); with self-gravity SubStep1's vri and vti are k_sources' inputs
+  k.e_mid = k.trr;
+  k.vr_mid = p->self_gravity ? k.tpp : k.vri;
+  k.vt_mid = p->self_gravity ? k.trp : k.vti;
   {
     // the CFL kernel leaves one set of force/mass partials per ring
     const int nb = nr;
@@ -542,6 +551,7 @@ extern "C" int fb_create(const fb_params *p, const double *radii, fb_ctx **out)
   {
     const char *cap = getenv("FB_MAX_SUBSTEPS");
     if (cap && atoi(cap) > 0) ctx->substep_cap = atoi(cap);
+    k.cap = ctx->substep_cap;
   }
   if (getenv("FB_NO_GRAPH")) ctx->graph_state = -1;
   if (p->nbpart > 0) {
@@ -749,10 +759,12 @@ static int enqueue_substep(fb_ctx *ctx)
   }
   if (k.energy) STAGE(ST_SOUND, 1, fb_launch_soundspeed(k, k.visc_mode == 1, s));
   if (k.lsa && !k.corot) STAGE(ST_POT, 2, fb_launch_lsa_modes(k, s));  // the turbulent modes at the substep's start
-  STAGE(ST_POT, 1, fb_launch_potential(k, s));
+  // the potential with the turbulent modes, or beside the self-gravity branch;
+  // else k_sources evaluates it
+  if (k.lsa || k.self_gravity) STAGE(ST_POT, 1, fb_launch_potential(k, s));
   if (k.lsa) STAGE(ST_POT, 1, fb_launch_lsa_add(k, s));
-  STAGE(ST_SUB1, 1, fb_launch_substep1(k, s));
   if (k.self_gravity) {
+    STAGE(ST_SUB1, 1, fb_launch_substep1(k, s));
     if (sg_branch) {
       cudaStreamWaitEvent(s, ctx->ev_sg_done, 0);
     } else {
@@ -760,34 +772,32 @@ static int enqueue_substep(fb_ctx *ctx)
       STAGE(ST_SGCOLS, 1, fb_sg_cols(ctx->sg, s));
       STAGE(ST_SGINV, 1, fb_sg_rows_inv(ctx->sg, k, k.rho, s));
     }
-    STAGE(ST_SGUPD, 1, fb_sg_update_velocities(k, s));
   }
-  if (k.visc_mode) {
-    STAGE(ST_VTERMS, 1, fb_launch_viscous_terms(k, k.vri, k.vti, s));
-    STAGE(ST_VUPDATE, 1, fb_launch_viscous_update(k, k.vri, k.vti, 0.0, s));
-  }
-  STAGE(ST_SUB2, 1, fb_launch_substep2(k, s));
+  STAGE(ST_SRC, 1, fb_launch_sources(k, s));
+  KP kt = k;  // the transport takes the velocities the source terms left
+  kt.vr_src = k.vr_mid;
+  kt.vt_src = k.vt_mid;
   // the tile variant's ring means of vtheta, which SubStep2 has just
   // written for the last time before the transport: on a branch beside
   // SubStep3 and the radial pass (in line when profiling stage by stage)
-  const bool vm_branch = !ctx->profiling && fb_azi_launches(k) == 2;
+  const bool vm_branch = !ctx->profiling && fb_azi_launches(kt) == 2;
   if (vm_branch) {
     cudaEventRecord(ctx->ev_vm_fork, s);
     cudaStreamWaitEvent(ctx->st_sg, ctx->ev_vm_fork, 0);
-    fb_launch_azi_vmed(k, 0.0, ctx->st_sg);
+    fb_launch_azi_vmed(kt, 0.0, ctx->st_sg);
     cudaEventRecord(ctx->ev_vm_done, ctx->st_sg);
     ctx->launches += 1;
     ctx->pcount[ST_TVMED] += 1;
   }
   if (k.energy) STAGE(ST_SUB3, 1, fb_launch_substep3(k, s));  // with the stresses of the new velocities
-  STAGE(ST_TRAD, 1, fb_launch_transport_radial(k, 0.0, s));
+  STAGE(ST_TRAD, 1, fb_launch_transport_radial(kt, 0.0, s));
   if (vm_branch) {
     cudaStreamWaitEvent(s, ctx->ev_vm_done, 0);
-    STAGE(ST_TAZI, 1, fb_launch_transport_azimuthal(k, 0.0, s, true));
+    STAGE(ST_TAZI, 1, fb_launch_transport_azimuthal(kt, 0.0, s, true));
   } else {
     // the tile variant's ring means as a stage of their own, then the pass
-    if (fb_azi_launches(k) == 2) STAGE(ST_TVMED, 1, fb_launch_azi_vmed(k, 0.0, s));
-    STAGE(ST_TAZI, 1, fb_launch_transport_azimuthal(k, 0.0, s, true));
+    if (fb_azi_launches(kt) == 2) STAGE(ST_TVMED, 1, fb_launch_azi_vmed(kt, 0.0, s));
+    STAGE(ST_TAZI, 1, fb_launch_transport_azimuthal(kt, 0.0, s, true));
   }
   STAGE(ST_TVR, 1, fb_launch_transport_vr(k, s));
   if (k.open_inner || k.non_reflecting) {
@@ -820,7 +830,7 @@ static int enqueue_dt_prelude(fb_ctx *ctx)
     // the self-gravity field (SoftWriting = No), which sets the RadSGAcc /
     // AziSGAcc grids the first substep's particles read
     fb_sg_accel(ctx->sg, k, k.rho, s);
-    fb_sg_update_velocities(k, s, 1);
+    fb_sg_refresh(k, s);
     n += fb_sg_launches(ctx->sg);
   }
   if (k.energy) {  // SourceEuler.c:344-350
@@ -1597,7 +1607,7 @@ extern "C" int fb_tune(fb_ctx *ctx, int substeps, fb_tuning *best, double *ms_ou
   Snapshot sn;
   rc = snapshot_take(ctx, sn);
   if (rc) { snapshot_free(sn); fb_profile(ctx, 0); return rc; }
-  const int cell_stages[] = {ST_POT, ST_SUB1, ST_VTERMS, ST_VUPDATE, ST_SUB2, ST_SUB3, ST_TVR};
+  const int cell_stages[] = {ST_POT, ST_SUB1, ST_SUB3, ST_TVR};
   const int azi_stage[] = {ST_TAZI};
   const int rad_stage[] = {ST_TRAD};
   double total = 0.0;
@@ -1608,7 +1618,7 @@ extern "C" int fb_tune(fb_ctx *ctx, int substeps, fb_tuning *best, double *ms_ou
     double bestms = 1e300;
     for (int c : cand) {
       k.cell_bs = c;
-      const double ms = tune_measure(ctx, sn, substeps, cell_stages, 7);
+      const double ms = tune_measure(ctx, sn, substeps, cell_stages, 4);
       if (ms >= 0.0 && ms < bestms) { bestms = ms; bestv = c; }
     }
     k.cell_bs = bestv;

@@ -72,6 +72,8 @@ struct fb_lsa {
   double s[FB_LSA_MAX_MODES], cp[FB_LSA_MAX_MODES], sp[FB_LSA_MAX_MODES];
 };
 
+#define FB_SRC_TAB 14  // doubles per ring of KP::src_tab
+
 // Everything a kernel needs, passed by value (well under the 32 KB limit).
 struct KP {
   int nr, ns;
@@ -84,6 +86,11 @@ struct KP {
   double *divv, *trr, *tpp, *trp, *vischeat;
   double *q[6];        // transport: RadMomP, RadMomM, ThetaMomP, ThetaMomM, Energy, Rho
   double *rho_t;       // density after transport, before floors
+  // the velocities and the energy the source terms leave (scratch fields); the
+  // transport reads its velocities from vr_src and vt_src (NULL: vr and vt,
+  // the transport on its own)
+  double *vr_mid, *vt_mid, *e_mid;
+  const double *vr_src, *vt_src;
   // tile variant of the azimuthal pass: RadMomP and RadMomM after the radial
   // pass and a copy of vtheta (three fields), and the ring means of vtheta
   // (nr); vt_copy is azt_buf[2] in the radial pass feeding the tile variant,
@@ -93,6 +100,7 @@ struct KP {
   double *lost0;       // ns: ring-0 radial mass fluxes of the last substep
   double *sg_accr, *sg_acct;  // SG accelerations (nf)
   // per-ring tables (nr or nr+1 entries)
+  const double *src_tab;   // the ring entries k_sources reads, FB_SRC_TAB per ring (fb_source_table)
   const double *rinf, *rsup, *rmed, *surf, *invrmed, *invsurf, *invdiffrsup, *invrinf, *invdiffrmed;
   const double *cosaz, *sinaz;
   const double *cs_ring;   // isothermal sound speed per ring
@@ -114,10 +122,11 @@ struct KP {
   double vh_l1, vh_l2;     // log(r/rip), log(rip/ri2p) for ViscHeat at i=0
   // CFL / reductions
   double *ringmin, *vmoy;
-  double *vt_part;  // beta cooling: per ring, SubStep2's partial sums of vtheta (one per CTA)
+  double *vt_part;  // beta cooling: per ring, SubStep2's partial sums of vtheta (one per tile of k_sources)
   double *partials;
   int n_partial_blocks;
   fb_ctl *ctl;
+  int cap;  // most substeps of a DT
   // scalars
   double pmin, pmax, dphi, invdphi, omega_frame;
   // frame corotating with the first planet (FRAME C): OmegaFrame changes
@@ -344,6 +353,13 @@ void fb_launch_planets(const KP &k, const PP *pp, cudaStream_t s);
 void fb_launch_correct_vtheta(const KP &k, cudaStream_t s);  // corotating frame: CorrectVtheta
 void fb_launch_soundspeed(const KP &k, int update_gcs, cudaStream_t s);
 void fb_launch_potential(const KP &k, cudaStream_t s);
+// the source terms in one pass (fb_source.cu): potential, SubStep1, the
+// self-gravity kicks, viscosity and SubStep2, from the state to vr_mid, vt_mid
+// and e_mid; with self-gravity the potential and SubStep1 come before it
+void fb_launch_substep1(const KP &k, cudaStream_t s);
+void fb_launch_sources(const KP &k, cudaStream_t s);
+int  fb_source_tiles(int ns);  // partial sums of vtheta per ring (KP::vt_part)
+void fb_source_table(const fb_geom *g, const double *invdxtheta, const double *p15, const double *cs_ring, double *out);
 // turbulent potential: mode draws and tables after the controller, the
 // modes' sum added to the potential after k_potential (two and one launches)
 void fb_launch_lsa_modes(const KP &k, cudaStream_t s);
@@ -355,10 +371,8 @@ int fb_launch_opacity_now(const KP &k, cudaStream_t s);
 int fb_launch_substep0(const KP &k, cudaStream_t s);
 int fb_launch_td_cfl(const KP &k, cudaStream_t s);  // explicit radiative diffusion's CFL limits
 int fb_sor_grid(void);  // CTAs of the solver kernel the GPU holds at once
-void fb_launch_substep1(const KP &k, cudaStream_t s);
 void fb_launch_viscous_terms(const KP &k, const double *vr, const double *vt, cudaStream_t s);
 void fb_launch_viscous_update(const KP &k, double *vr, double *vt, double dt_override, cudaStream_t s);
-void fb_launch_substep2(const KP &k, cudaStream_t s);
 void fb_launch_substep3(const KP &k, cudaStream_t s);
 void fb_launch_transport(const KP &k, double dt_override, cudaStream_t s);
 void fb_launch_transport_radial(const KP &k, double dt_override, cudaStream_t s);
@@ -393,8 +407,8 @@ struct fb_sg;
 int  fb_sg_create(fb_sg **out, const fb_params *p, const fb_geom *g, cudaStream_t s);
 void fb_sg_destroy(fb_sg *sg);
 void fb_sg_accel(fb_sg *sg, const KP &k, const double *dens, cudaStream_t s);
-// refresh = 1: the Dt = 0 call of main.c:316 on Vrad/Vtheta (fields only)
-void fb_sg_update_velocities(const KP &k, cudaStream_t s, int refresh = 0);
+// the Dt = 0 call of main.c:316 on Vrad/Vtheta: the particles' RadSGAcc / AziSGAcc grids
+void fb_sg_refresh(const KP &k, cudaStream_t s);
 // context accessors for the other modules (fb_api.cu)
 const KP *fb_ctx_kp(const fb_ctx *ctx);
 KP *fb_ctx_kp_mut(fb_ctx *ctx);

@@ -712,7 +712,8 @@ static __device__ __forceinline__ double pressure_at(const KP &k, size_t l)
   return (k.gamma - 1.0) * k.e[l];
 }
 
-// SubStep1 (SourceEuler.c:765-1009) without dust: pressure, potential and
+// With self-gravity (k_sources evaluates it otherwise): SubStep1
+// (SourceEuler.c:765-1009) without dust: pressure, potential and
 // curvature terms into VradInt (i >= 1) and VthetaInt (all rings).  At most
 // 64 registers, so that four 256-thread CTAs share an SM (68 would allow three).
 __global__ void __launch_bounds__(FB_BS2, 4) k_substep1(KP k)
@@ -720,6 +721,7 @@ __global__ void __launch_bounds__(FB_BS2, 4) k_substep1(KP k)
   fb_grid_dependency();
   const int ns = k.ns;
   const double dt = k.ctl->dt;
+  const bool keep = k.ctl->done || k.ctl->status || k.ctl->substeps >= k.cap;
   const int i = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= ns) return;
   const size_t l = (size_t)i * ns + j;
@@ -750,7 +752,7 @@ __global__ void __launch_bounds__(FB_BS2, 4) k_substep1(KP k)
     ipjm = k.indpot[ljm];
     if (i >= 1) iplim = k.indpot[lim];
   }
-  k.pres[l] = Pl;
+  if (keep) k.pres[l] = Pl;  // nothing but fb_download_derived reads it
   if (i >= 1) {
     double gradp = (Pl - Plim) * 2.0 / (rl + rlim) * invdiffrmed;
     double gradphi = (potl - potlim) * invdiffrmed;
@@ -891,91 +893,6 @@ void fb_launch_viscous_update(const KP &k, double *vr, double *vt, double dt_ove
   fb_launch(k_viscous_update, grid2d(k, k.nr), k.cell_bs, 0, s, k, vr, vt, dt_override);
 }
 
-// ------------------------------------------------------------ SubStep2
-// SubStep2 (SourceEuler.c:1012-1116) followed by the copies of
-// SourceEuler.c:617-622: artificial viscosity from VradInt/VthetaInt into
-// Vrad/Vtheta (and EnergyInt into Energy).  Rings the reference never
-// writes in VradNew/VthetaNew/EnergyInt (ring 0 and ring nr of VradNew, ring
-// nr of the others) are zero, and the copies spread those zeros.
-static __device__ __forceinline__ double q_r(const KP &k, size_t l, size_t lip)
-{
-  double dv = k.vri[lip] - k.vri[l];
-  return (dv < 0.0) ? FB_CVNR * FB_CVNR * k.rho[l] * dv * dv : 0.0;
-}
-static __device__ __forceinline__ double q_t(const KP &k, size_t l, size_t ljp)
-{
-  double dv = k.vti[ljp] - k.vti[l];
-  return (dv < 0.0) ? FB_CVNR * FB_CVNR * k.rho[l] * dv * dv : 0.0;
-}
-
-// At most 48 registers: five 256-thread CTAs per SM (SubStep2 20.6 -> 19.0 us;
-// the same cap made the stress kernels and SubStep3 slower).
-__global__ void __launch_bounds__(FB_BS2, 5) k_substep2(KP k)
-{
-  fb_grid_dependency();
-  const int ns = k.ns, nr = k.nr;
-  const double dt = k.ctl->dt;
-  const int i = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool cell = (j < ns);
-  const size_t l = (size_t)i * ns + j;
-  if (i == nr) {  // the whole CTA
-    if (!cell) return;
-    k.vr[l] = 0.0;
-    k.vt[l] = 0.0;
-    if (k.energy) k.e[l] = 0.0;
-    return;
-  }
-  double vtnew = 0.0;
-  if (cell) {
-    const size_t lip = l + ns;
-    const size_t ljp = (j == ns - 1) ? (size_t)i * ns : l + 1;
-    const size_t ljm = (j == 0) ? (size_t)i * ns + ns - 1 : l - 1;
-    const size_t lim = (i >= 1) ? l - ns : l;
-    // every load first
-    const double qr = q_r(k, l, lip);
-    const double qt = q_t(k, l, ljp);
-    const double qtjm = q_t(k, ljm, l);
-    const double qrim = (i >= 1) ? q_r(k, lim, l) : 0.0;
-    const double rl = k.rho[l], rlim = k.rho[lim], rjm = k.rho[ljm];
-    const double vril = k.vri[l], vtil = k.vti[l];
-    const double invdxtheta = k.invdxtheta[i], invdiffrmed = k.invdiffrmed[i];
-    double el = 0.0, vrip = 0.0, vtijp = 0.0, invdiffrsup = 0.0;
-    if (k.energy) {
-      el = k.e[l];
-      vrip = k.vri[lip];
-      vtijp = k.vti[ljp];
-      invdiffrsup = k.invdiffrsup[i];
-    }
-    if (i >= 1)
-      k.vr[l] = vril - dt * 2.0 / (rl + rlim) * (qr - qrim) * invdiffrmed;
-    else
-      k.vr[l] = 0.0;
-    vtnew = vtil - dt * 2.0 / (rl + rjm) * (qt - qtjm) * invdxtheta;
-    k.vt[l] = vtnew;
-    if (k.energy)
-      k.e[l] = el - dt * qr * (vrip - vril) * invdiffrsup - dt * qt * (vtijp - vtil) * invdxtheta;
-  }
-  if (k.energy && k.beta_cooling) {
-    // SubStep3's ring mean of vtheta (SourceEuler.c:1196-1203): this CTA's
-    // part, summed in a fixed order
-    __shared__ double sh[FB_BS2 / 32];
-    double v = cell ? (vtnew + k.rmed[i] * omf(k)) : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sh[w];
-      k.vt_part[(size_t)i * gridDim.x + blockIdx.x] = t;
-    }
-  }
-}
-
-void fb_launch_substep2(const KP &k, cudaStream_t s)
-{
-  fb_launch(k_substep2, grid2d(k, k.nr + 1), k.cell_bs, 0, s, k);
-}
-
 // ------------------------------------------------------------ SubStep3
 static __device__ __forceinline__ double vischeat_of(const KP &k, int i, double rho, const Stress &st)
 {
@@ -995,48 +912,48 @@ static __device__ __forceinline__ double vischeat_of(const KP &k, int i, double 
 // one pass: a cell's stresses feed its own heating, so they are evaluated
 // here (and still stored) instead of read back.  Ring 0's heating is
 // extrapolated from rings 1 and 2, whose stresses its threads evaluate too.
-// Writes Energy = EnergyNew (ring nr of EnergyNew is never written: zero).
-__global__ void __launch_bounds__(FB_BS2) k_substep3(KP k)
+// Reads the velocities and the energy that k_sources left and writes Energy =
+// EnergyNew (ring nr stays zero).  DivV and the heating are stored by the last
+// substep of a DT only: nothing but fb_download_derived reads them.
+__global__ void __launch_bounds__(FB_BS2) k_substep3(KP k, int nparts)
 {
   fb_grid_dependency();
   const int ns = k.ns, nr = k.nr;
   const int i = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
+  // the ring sum of vtheta from the tiles' partial sums, by each warp in the
+  // same order (a lane's strided sums, then across lanes)
+  double vsum = 0.0;
+  if (k.beta_cooling) {
+    for (int b = threadIdx.x & 31; b < nparts; b += 32) vsum += k.vt_part[(size_t)i * nparts + b];
+    for (int o = 16; o > 0; o >>= 1) vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
+  }
   if (j >= ns) return;
   const size_t l = (size_t)i * ns + j;
-  if (i == nr) {
-    k.e[l] = 0.0;
-    return;
-  }
   const bool heat = k.viscous_heating;
-  const Stress st = stress_at(k, k.vr, k.vt, i, j, heat);
+  const Stress st = stress_at(k, k.vr_mid, k.vt_mid, i, j, heat);
   Stress s1, s2;
   double r1 = 0.0, r2 = 0.0;
   if (heat && i == 0) {
-    s1 = stress_at(k, k.vr, k.vt, 1, j, true);
-    s2 = stress_at(k, k.vr, k.vt, 2, j, true);
+    s1 = stress_at(k, k.vr_mid, k.vt_mid, 1, j, true);
+    s2 = stress_at(k, k.vr_mid, k.vt_mid, 2, j, true);
     r1 = k.rho[l + ns];
     r2 = k.rho[l + 2 * ns];
   }
-  const double el = k.e[l], rl = k.rho[l];
+  const double el = k.e_mid[l], rl = k.rho[l];
   const double dt = k.ctl->dt;
+  const bool keep = k.ctl->done || k.ctl->status || k.ctl->substeps >= k.cap;
   double coolfac = 0.0;
   if (k.beta_cooling) {
-    // the ring mean of vtheta from SubStep2's partial sums (same CTA width)
-    double s = 0.0;
-    for (int b = 0; b < (int)gridDim.x; b++) s += k.vt_part[(size_t)i * gridDim.x + b];
-    double omega = s;
+    double omega = vsum;
     omega /= (double)ns;
     omega /= k.rmed[i];
     double coolingtime = k.betatab[i] / omega;
     coolfac = coolingtime;
   }
-  k.divv[l] = st.div;
+  if (keep) k.divv[l] = st.div;
   double vh = 0.0;
   if (heat) {
-    k.trr[l] = st.trr;
-    k.tpp[l] = st.tpp;
     if (i >= 1) {
-      k.trp[l] = st.trp;
       vh = vischeat_of(k, i, rl, st);
     } else {
       // the i = 0 extrapolation tests the viscosity of the last ring visited
@@ -1046,7 +963,7 @@ __global__ void __launch_bounds__(FB_BS2) k_substep3(KP k)
       const double qpi2p = vischeat_of(k, 2, r2, s2);
       vh = (visc_last != 0.0) ? qpip * exp(log(qpip / qpi2p) * k.vh_l1 / k.vh_l2) : 0.0;
     }
-    k.vischeat[l] = vh;
+    if (keep) k.vischeat[l] = vh;
   }
   const double dv = st.div;
   double en;
@@ -1159,7 +1076,10 @@ int fb_launch_opacity_now(const KP &k, cudaStream_t s)
   return 1;
 }
 
-void fb_launch_substep3(const KP &k, cudaStream_t s) { fb_launch(k_substep3, grid2d(k, k.nr + 1), k.cell_bs, 0, s, k); }
+void fb_launch_substep3(const KP &k, cudaStream_t s)
+{
+  fb_launch(k_substep3, grid2d(k, k.nr), k.cell_bs, 0, s, k, fb_source_tiles(k.ns));
+}
 
 // ------------------------------------------------------------ Transport
 // Radial pass of the van Leer transport (OneWindRad, TransportEuler.c:124-220
@@ -1208,16 +1128,16 @@ static __device__ __forceinline__ void radial_column(const KP &k, double dt, int
       const size_t l = (size_t)kk * ns + j;
       w.r = k.rho[l];
       if (H == 0) {
-        w.u0 = k.vr[l + ns];
-        w.u1 = k.vr[l];
-        w.u2 = k.vt[(size_t)kk * ns + jp];
+        w.u0 = k.vr_src[l + ns];
+        w.u1 = k.vr_src[l];
+        w.u2 = k.vt_src[(size_t)kk * ns + jp];
       } else {
-        w.u0 = k.vt[l];
+        w.u0 = k.vt_src[l];
         if (NQ == 6) w.u1 = k.e[l];
         if (k.vt_copy && kk >= i0 && kk < i1) k.vt_copy[l] = w.u0;  // for the tile variant
       }
     }
-    if (kk >= 0 && kk <= nr) w.v = k.vr[(size_t)kk * ns + j];
+    if (kk >= 0 && kk <= nr) w.v = k.vr_src[(size_t)kk * ns + j];
     return w;
   };
   auto put = [&](const Raw &w, int kk, int slot) {
@@ -1414,7 +1334,7 @@ __global__ void __launch_bounds__(AziMaxThreads<E, WIDE>::value) k_transport_azi
   const double invdt = 1.0 / dt;
   double s = 0.0;
   for (int j = tid; j < ns; j += T) {
-    double elong = k.vt[base + j] * dt;
+    double elong = k.vt_src[base + j] * dt;
     s += elong * invdt;
   }
   s = block_sum_dyn(s, sh);
@@ -1426,7 +1346,7 @@ __global__ void __launch_bounds__(AziMaxThreads<E, WIDE>::value) k_transport_azi
   const long nshift = (long)Nround;
   double vconst = (Ntilde - Nround) * k.rmed[i] * invdt * dpinvns;
   for (int j = tid; j < ns; j += T) {
-    double elong = k.vt[base + j] * dt;
+    double elong = k.vt_src[base + j] * dt;
     double v = elong * invdt - VMed;
     if (!k.fast_transport) v = vconst + v;
     vres[j] = v;
@@ -1662,8 +1582,8 @@ __global__ void __launch_bounds__((E == 1) ? 1024 : 768) k_transport_azimuthal_p
       if (!OWN(e)) continue;
 #pragma unroll
       for (int q = 0; q < AZP; q++) v[e][q] = (q < NQ) ? k.q[q][base + jj[e]] : 0.0;
-      vtc[e] = k.vt[base + jj[e]];
-      vtn[e] = k.vt[base + jjp[e]];
+      vtc[e] = k.vt_src[base + jj[e]];
+      vtn[e] = k.vt_src[base + jjp[e]];
     }
 #pragma unroll
     for (int e = 0; e < E; e++) {
@@ -2168,9 +2088,9 @@ __global__ void __launch_bounds__(MT) k_transport_azimuthal_reg(KP k, double dto
   double q0[NQ][E], vt[E], vs[E];
 #pragma unroll
   for (int q = 0; q < NQ; q++) azr_load<E>(k.q[q] + base + c0, q0[q]);
-  azr_load<E>(k.vt + base + c0, vt);
+  azr_load<E>(k.vt_src + base + c0, vt);
 #pragma unroll
-  for (int e = 0; e < E; e++) vs[e] = k.vt[base + tid + e * T];
+  for (int e = 0; e < E; e++) vs[e] = k.vt_src[base + tid + e * T];
   const AzrTab tb = azr_tab(k, i);
   azr_ring<NQ, E, false>(k, dt, i, tb, q0, vt, vs, 0.0, c0, sh, hal, xb,
                          [&](int, int p, double v, double r, double a, double b, double en) {
@@ -2209,7 +2129,7 @@ __global__ void __launch_bounds__(1024) k_azi_vmed(KP k, double dtov)
   __shared__ double sh[32];
   const double dt = dt_of(k, dtov);
   const int i = blockIdx.x, ns = k.ns, T = blockDim.x;
-  const double *vt = k.vt + (size_t)i * ns;
+  const double *vt = k.vt_src + (size_t)i * ns;
   const double invdt = 1.0 / dt;
   double s = 0.0;
   for (int j = threadIdx.x; j < ns; j += T) {
@@ -2242,7 +2162,7 @@ __global__ void __launch_bounds__(AZT_WPC * 32, MINB) k_transport_azimuthal_tile
     const size_t l = base + g;
 #pragma unroll
     for (int q = 0; q < NQ; q++) q0[q][e] = (q < 2 ? k.azt_buf[q] : k.q[q])[l];
-    vt[e] = k.azt_buf[2][l];
+    vt[e] = k.vt_src[l];
     vs[e] = 0.0;
   }
   const AzrTab tb = azr_tab(k, i);
@@ -2328,7 +2248,7 @@ __global__ void __launch_bounds__(MT) k_transport_azimuthal_staged(KP k, double 
     azs_expect(&bar[b], NB * row_bytes);
 #pragma unroll
     for (int q = 0; q < NQ; q++) azs_load(buf + (size_t)(b * NB + q) * ns, k.q[q] + base, row_bytes, &bar[b]);
-    azs_load(buf + (size_t)(b * NB + NQ) * ns, k.vt + base, row_bytes, &bar[b]);
+    azs_load(buf + (size_t)(b * NB + NQ) * ns, k.vt_src + base, row_bytes, &bar[b]);
   };
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(azs_smem(&bar[0])) : "memory");
@@ -2450,7 +2370,7 @@ static bool azs_fits(int ns, int energy, int E)
 static bool azs_pointers_aligned(const KP &k, int NQ)
 {
   auto al = [](const void *p) { return ((unsigned long long)p & 15ull) == 0; };
-  bool ok = al(k.vt) && al(k.rho_t) && (NQ != 6 || al(k.e));
+  bool ok = al(k.vt) && al(k.vt_src ? k.vt_src : k.vt) && al(k.rho_t) && (NQ != 6 || al(k.e));
   for (int q = 0; q < NQ; q++) ok = ok && al(k.q[q]);
   return ok;
 }
@@ -2545,7 +2465,7 @@ __global__ void __launch_bounds__(FB_BS2) k_transport_vr(KP k)
       const size_t m = (size_t)ii * ns + j;
       return (k.q[0][m - ns] + k.q[1][m]) / (k.rho_t[m] + k.rho_t[m - ns] + 1e-20);
     };
-    if (i == nr) {
+    if (i == nr) {  // zero without the wall since SubStep2 (k_sources)
       if (wall) k.vr[l] = -vr_at(nr - 2);
       return;
     }
@@ -2622,16 +2542,26 @@ int fb_rad_chunk_auto(const KP &k)
   return best;
 }
 
+// The transport's velocities: those the source terms left, else the state's.
+static KP with_sources(const KP &k0)
+{
+  KP k = k0;
+  if (!k.vr_src) k.vr_src = k.vr;
+  if (!k.vt_src) k.vt_src = k.vt;
+  return k;
+}
+
 void fb_launch_transport_radial(const KP &k0, double dt_override, cudaStream_t s)
 {
-  // before the tile variant: RadMomP, RadMomM and a copy of vtheta into its
-  // scratch fields (it cannot update them in place)
-  KP k = k0;
+  // before the tile variant: RadMomP and RadMomM into its scratch fields,
+  // and a copy of vtheta where the pass would read it from vt itself (it
+  // cannot update them in place)
+  KP k = with_sources(k0);
   k.vt_copy = nullptr;
   if (azt_variant(azi_resolve(k0, nullptr))) {
     k.q[0] = k0.azt_buf[0];
     k.q[1] = k0.azt_buf[1];
-    k.vt_copy = k0.azt_buf[2];
+    if (!k0.vt_src) k.vt_copy = k0.azt_buf[2];
   }
   const int tx = k.rad_tx > 0 ? k.rad_tx : 64, bx = (k.ns + tx - 1) / tx;
   const int chunk = k.rad_chunk > 0 ? k.rad_chunk : fb_rad_chunk_auto(k);
@@ -2645,19 +2575,22 @@ void fb_launch_transport_radial(const KP &k0, double dt_override, cudaStream_t s
 // The tile variant's ring means of vtheta (k_azi_vmed): nothing between
 // SubStep2 and the azimuthal pass changes vtheta, so the step may run them
 // on a branch beside SubStep3 and the radial pass.  Returns the launches.
-int fb_launch_azi_vmed(const KP &k, double dt_override, cudaStream_t s)
+int fb_launch_azi_vmed(const KP &k0, double dt_override, cudaStream_t s)
 {
   int E = 1;
-  if (!azt_variant(azi_resolve(k, &E))) return 0;
+  if (!azt_variant(azi_resolve(k0, &E))) return 0;
+  const KP k = with_sources(k0);
   fb_launch(k_azi_vmed, k.nr, azi_threads_for(k.ns, E), 0, s, k, dt_override);
   return 1;
 }
 
 template <int NQ>
-static void launch_azimuthal(const KP &k, double dt_override, cudaStream_t s, bool vmed_done)
+static void launch_azimuthal(const KP &k0, double dt_override, cudaStream_t s, bool vmed_done)
 {
   int E = 1;
-  const int var = azi_resolve(k, &E);
+  const int var = azi_resolve(k0, &E);
+  KP k = with_sources(k0);
+  if (azt_variant(var) && !k0.vt_src) k.vt_src = k0.azt_buf[2];  // the radial pass's copy
   const bool wide = (var == 2);
   const int th = azi_threads_for(k.ns, E);
   const bool full = (th * E == k.ns);  // every thread owns E cells

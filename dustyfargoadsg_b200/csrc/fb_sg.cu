@@ -22,7 +22,7 @@
 //   3. sg_rows_inv : per ring, one inverse complex FFT of Wr + i Wt (both
 //      Hermitian), whose real and imaginary parts are the two accelerations,
 //      with the normalisation and self-force term of sgacc.c:138-161 fused;
-//   4. sg_update   : the velocity kicks of update_sgvelocity (sgupdate.c).
+// The velocity kicks of update_sgvelocity (sgupdate.c) are part of k_sources.
 // The kernel spectra are computed once (host glibc for K, device FFT).
 #include <cuda_runtime.h>
 #include <math.h>
@@ -819,40 +819,22 @@ __global__ void __launch_bounds__(SG_ROW_BS, 4) sg_rows_inv(FftArgs fa, int ns, 
   }
 }
 
-// update_sgvelocity (sgupdate.c:30-72) on VradInt / VthetaInt.  refresh = 1
-// is the call the reference's main loop makes before every DT
-// (main.c:316, Dt = 0, on Vrad / Vtheta), which matters only for the
-// RadSGAcc / AziSGAcc grids the particles read.
-__global__ void __launch_bounds__(SG_BS) sg_update(KP k, int refresh)
+// update_sgvelocity (sgupdate.c:30-72) as the reference's main loop calls it
+// before every DT (main.c:316, Dt = 0, which leaves the velocities alone):
+// the RadSGAcc / AziSGAcc grids the particles read.  The substep's own kicks
+// are part of k_sources.
+__global__ void __launch_bounds__(SG_BS) sg_refresh(KP k)
 {
   fb_grid_dependency();
   const int ns = k.ns;
   const int i = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= ns) return;
-  const double Dt = refresh ? 0.0 : k.ctl->dt;
-  double *vr = refresh ? k.vr : k.vri;
-  double *vt = refresh ? k.vt : k.vti;
   const size_t l = (size_t)i * ns + j;
   const size_t lm1 = (size_t)i * ns + (j == 0 ? ns - 1 : j - 1);
-  // every load first
-  const double at0 = k.sg_acct[l], at1 = k.sg_acct[lm1], vtl = vt[l];
-  double ar0 = 0.0, ar1 = 0.0, vrl = 0.0, c0 = 0.0, c1 = 0.0, invd = 0.0;
-  if (i > 0) {
-    ar0 = k.sg_accr[l];
-    ar1 = k.sg_accr[l - ns];
-    vrl = vr[l];
-    c0 = k.rinf[i] - k.rmed[i - 1];
-    c1 = k.rmed[i] - k.rinf[i];
-    invd = k.invdiffrmed[i];
-  }
-  if (i > 0) {
-    const double radsgacc = (c0 * ar0 + c1 * ar1) * invd;
-    vr[l] = vrl + Dt * radsgacc;
-    if (k.particles) k.rsga[l] = radsgacc;
-  }
-  const double azisgacc = 0.5 * (at0 + at1);
-  vt[l] = vtl + Dt * azisgacc;
-  if (k.particles) k.asga[l] = azisgacc;
+  if (i > 0)
+    k.rsga[l] = ((k.rinf[i] - k.rmed[i - 1]) * k.sg_accr[l] + (k.rmed[i] - k.rinf[i]) * k.sg_accr[l - ns]) *
+                k.invdiffrmed[i];
+  k.asga[l] = 0.5 * (k.sg_acct[l] + k.sg_acct[lm1]);
 }
 
 // ------------------------------------------------------------------- host
@@ -1019,9 +1001,9 @@ void fb_sg_accel(fb_sg *sg, const KP &k, const double *dens, cudaStream_t s)
   fb_sg_rows_inv(sg, k, dens, s);
 }
 
-void fb_sg_update_velocities(const KP &k, cudaStream_t s, int refresh)
+void fb_sg_refresh(const KP &k, cudaStream_t s)
 {
-  fb_launch(sg_update, dim3((k.ns + SG_BS - 1) / SG_BS, k.nr), SG_BS, 0, s, k, refresh);
+  fb_launch(sg_refresh, dim3((k.ns + SG_BS - 1) / SG_BS, k.nr), SG_BS, 0, s, k);
 }
 
 int fb_sg_launches(const fb_sg *sg) { return sg ? 4 : 0; }
