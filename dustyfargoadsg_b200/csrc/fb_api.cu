@@ -11,12 +11,12 @@
 
 #define FB_PROFILE_POINTS 64
 enum {
-  ST_CFL, ST_SUB0, ST_SOUND, ST_POT, ST_SUB1, ST_SG, ST_SGCOLS, ST_SGINV, ST_SRC, ST_SUB3, ST_TRAD, ST_TAZI, ST_TVR, ST_DAMP, ST_DUST, ST_TVMED, FB_NSTAGE
+  ST_CFL, ST_SUB0, ST_SOUND, ST_POT, ST_SUB1, ST_SG, ST_SGCOLS, ST_SGINV, ST_SRC, ST_SUB3, ST_TRAD, ST_TAZI, ST_TVR, ST_DAMP, ST_FIN, ST_DUST, ST_TVMED, FB_NSTAGE
 };
 static const char *stage_names[FB_NSTAGE] = {
   "cfl_forces", "substep0", "soundspeed", "potential", "substep1", "sg_rows_fwd", "sg_cols", "sg_rows_inv",
   "source_terms", "substep3",
-  "transport_radial", "transport_azimuthal", "transport_vr_boundary", "damping", "dust_particles",
+  "transport_radial", "transport_azimuthal", "transport_vr_boundary", "damping", "finish", "dust_particles",
   "transport_ring_means"};
 
 struct fb_ctx {
@@ -699,11 +699,33 @@ extern "C" int fb_upload(fb_ctx *ctx, const fb_state *s, const fb_profiles *prof
     ctx->pcount[id] += (nlaunch);                                \
   } while (0)
 
-static int enqueue_substep(fb_ctx *ctx)
+// Two orders of the same steps.  A substep starts with its time step (k_cfl)
+// and ends with the damping; where the end of the substep is one kernel that
+// also takes the next substep's limits (cfl_at_end), the DT's prelude runs the
+// first k_cfl and the body starts behind it.  Self-gravity keeps k_cfl first,
+// where it runs beside the convolution; so do the discs whose edges or
+// opacities change between the damping and the limits, and large grids
+// (fb_finish_fits).
+static bool edges_other_than_wall(const KP &k) { return k.open_inner || k.non_reflecting; }
+static bool cfl_at_end(const KP &k)
+{
+  return !k.self_gravity && !edges_other_than_wall(k) && !(k.energy && k.rad_diff == 1) && fb_finish_fits(k);
+}
+// the next substep's sound speed with the limits: not where the particles'
+// update or the thermal diffusion come in between
+static bool cs_at_end(const fb_ctx *ctx)
+{
+  const KP &k = ctx->k;
+  return cfl_at_end(k) && k.energy && !ctx->has_dust && !k.ent_diff && !k.rad_diff;
+}
+static bool more_substeps(const fb_ctx *ctx) { return cfl_at_end(ctx->k) ? ctx->h_ctl->go : !ctx->h_ctl->done; }
+
+static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NULL)
 {
   KP &k = ctx->k;
   cudaStream_t s = ctx->st;
   int npt = 0;
+  const bool at_end = cfl_at_end(k), cs_done = cs_at_end(ctx);
   // The self-gravity convolution reads only the density, which no kernel
   // changes before the transport: outside the per-stage profile it runs on
   // a branch of its own from the start of the substep, beside the CFL,
@@ -728,7 +750,7 @@ static int enqueue_substep(fb_ctx *ctx)
     STAGE(ST_CFL, 1, fb_launch_opacity_now(k, s));
     STAGE(ST_CFL, 1, fb_launch_td_cfl(k, s));
   }
-  STAGE(ST_CFL, 1, fb_launch_cfl(k, s));  // ConditionCFL + the controller (last CTA)
+  if (!at_end) STAGE(ST_CFL, 1, fb_launch_cfl(k, s));  // ConditionCFL + the controller (last CTA)
   if (k.corot) {
     // corotating frame: FillForcesArrays' turbulent modes still see the old
     // OmegaFrame; then the planets' step sets the new one and CorrectVtheta
@@ -757,7 +779,7 @@ static int enqueue_substep(fb_ctx *ctx)
     int n0 = 0;  // the stage's kernel launches
     STAGE(ST_SUB0, n0, n0 = fb_launch_substep0(k, s));
   }
-  if (k.energy) STAGE(ST_SOUND, 1, fb_launch_soundspeed(k, k.visc_mode == 1, s));
+  if (k.energy && !cs_done) STAGE(ST_SOUND, 1, fb_launch_soundspeed(k, k.visc_mode == 1, s));
   if (k.lsa && !k.corot) STAGE(ST_POT, 2, fb_launch_lsa_modes(k, s));  // the turbulent modes at the substep's start
   // the potential with the turbulent modes, or beside the self-gravity branch;
   // else k_sources evaluates it
@@ -799,8 +821,8 @@ static int enqueue_substep(fb_ctx *ctx)
     if (fb_azi_launches(kt) == 2) STAGE(ST_TVMED, 1, fb_launch_azi_vmed(kt, 0.0, s));
     STAGE(ST_TAZI, 1, fb_launch_transport_azimuthal(kt, 0.0, s, true));
   }
-  STAGE(ST_TVR, 1, fb_launch_transport_vr(k, s));
-  if (k.open_inner || k.non_reflecting) {
+  if (!at_end) STAGE(ST_TVR, 1, fb_launch_transport_vr(k, s));
+  if (edges_other_than_wall(k)) {
     // ApplyBoundaryCondition's other edges (SideEuler.c:1102-1131); the
     // non-reflecting edge reads the planets' new positions and, with the
     // energy equation, the sound speed of the transported state
@@ -808,8 +830,14 @@ static int enqueue_substep(fb_ctx *ctx)
     if (k.non_reflecting && k.energy) STAGE(ST_TVR, 1, fb_launch_soundspeed(k, 0, s));
     STAGE(ST_TVR, 1, fb_launch_edges(k, s));
   }
-  if (k.evanescent && k.n_damp_rings > 0) STAGE(ST_DAMP, 1, fb_launch_damping(k, 0.0, s));
+  if (!at_end && k.evanescent && k.n_damp_rings > 0) STAGE(ST_DAMP, 1, fb_launch_damping(k, 0.0, s));
   if (!ctx->has_dust) cudaStreamWaitEvent(s, ctx->ev_planets, 0);
+  if (at_end) {
+    STAGE(ST_FIN, 1, fb_launch_finish(k, cs_done, h, s));
+  } else if (h) {
+    fb_launch_loop_cond(k, *h, ctx->substep_cap, s);
+    ctx->launches += 1;
+  }
   if (ctx->profiling) {
     cudaEventRecord(ctx->pev[npt], s);
     ctx->pseq[npt] = -1;
@@ -838,6 +866,14 @@ static int enqueue_dt_prelude(fb_ctx *ctx)
     n += 1;
   }
   if (ctx->has_dust) n += fb_launch_dust_sort(k, ctx->pp, s);  // processing order only
+  if (cfl_at_end(k)) {  // the first substep's limits and sound speed
+    fb_launch_cfl(k, s);
+    n += 1;
+    if (cs_at_end(ctx)) {
+      fb_launch_soundspeed(k, k.visc_mode == 1, s);
+      n += 1;
+    }
+  }
   return n;
 }
 
@@ -881,12 +917,11 @@ static int build_dt_graph_once(fb_ctx *ctx)
   ctx->profiling = 0;
   cudaError_t e = cudaStreamBeginCaptureToGraph(ctx->st, body, NULL, NULL, 0, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    enqueue_substep(ctx);
-    fb_launch_loop_cond(ctx->k, h, ctx->substep_cap, ctx->st);
+    enqueue_substep(ctx, &h);
     e = cudaStreamEndCapture(ctx->st, &body);
   }
   ctx->profiling = prof;
-  ctx->launches_per_substep = ctx->launches - l0 + 1;
+  ctx->launches_per_substep = ctx->launches - l0;
   ctx->launches = l0;
   for (int q = 0; q < FB_NSTAGE; q++) ctx->pcount[q] = 0;
   if (e != cudaSuccess) {
@@ -976,8 +1011,9 @@ extern "C" int fb_algogas(fb_ctx *ctx, fb_step_report *rep)
     CK(cudaMemcpyAsync(ctx->h_ctl, ctx->d_ctl, sizeof(fb_ctl), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     if (ctx->profiling) profile_collect(ctx, npt);
-    if (ctx->h_ctl->status) { status = ctx->h_ctl->status; break; }
-    if (ctx->h_ctl->done) break;
+    // (a status that the next substep's controller has set ends the loop behind that substep)
+    if (ctx->h_ctl->status && !(cfl_at_end(ctx->k) && ctx->h_ctl->go)) { status = ctx->h_ctl->status; break; }
+    if (!more_substeps(ctx)) break;
     if (it == cap - 1) status = FB_ERR_SUBSTEPS;
   }
   CK(cudaEventRecord(ctx->ev1, s));
@@ -1388,11 +1424,10 @@ static int batch_add_disc(fb_batch *b, fb_ctx *ctx)
     const long long l1 = ctx->launches;
     if (cudaStreamBeginCaptureToGraph(s, body, NULL, NULL, 0, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
       goto out;
-    enqueue_substep(ctx);
-    fb_launch_loop_cond(ctx->k, h, ctx->substep_cap, s);
+    enqueue_substep(ctx, &h);
     if (cudaStreamEndCapture(s, &body) != cudaSuccess) goto out;
     b->prelude.push_back(npre);
-    b->per_substep.push_back(ctx->launches - l1 + 1);
+    b->per_substep.push_back(ctx->launches - l1);
   }
   rc = FB_OK;
 out:
@@ -1589,7 +1624,7 @@ static double tune_measure(fb_ctx *ctx, const Snapshot &sn, int substeps, const 
     }
     profile_collect(ctx, npt);
     if (ctx->h_ctl->status) return -1.0;
-    if (ctx->h_ctl->done) enqueue_dt_prelude(ctx);  // start another DT from here
+    if (!more_substeps(ctx)) enqueue_dt_prelude(ctx);  // start another DT from here
   }
   ctx->launches = l0;
   double ms = 0.0;

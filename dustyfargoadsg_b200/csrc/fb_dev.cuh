@@ -24,6 +24,7 @@ struct fb_ctl {
   double bary_x[3], bary_y[3];               // stardiscbarycenter_{x,y}
   double mdisc;
   int substeps, done, status, nonfinite;
+  int go;                 // the loop runs another substep (k_finish; else it goes on while not done)
   // DetectCrash (SourceEuler.c:51-69) as AlgoGas uses it (:545-566): the
   // CFL kernel's CTAs raise the flags for the state at the start of the
   // substep, the controller consumes them.  Only the energy test decides a
@@ -387,6 +388,11 @@ void fb_launch_opacity(const KP &k, int constant, double imposed, double factor,
                        double unit_mass, double inv_l3, double conv, cudaStream_t s);
 void fb_launch_floors_boundary(const KP &k, cudaStream_t s);
 void fb_launch_damping(const KP &k, double dt_override, cudaStream_t s);
+// the end of a substep in one pass (discs with walls, small grids): vr, floors,
+// walls, damping, the next substep's CFL limits and controller, with fuse_cs
+// its sound speed, and the loop condition h (if any)
+int  fb_finish_fits(const KP &k);
+void fb_launch_finish(const KP &k, int fuse_cs, const cudaGraphConditionalHandle *h, cudaStream_t s);
 void fb_launch_diag(const KP &k, double *out2, cudaStream_t s);
 void fb_launch_derived(const KP &k, int which, double *out, cudaStream_t s);
 void fb_launch_boundary_only(const KP &k, cudaStream_t s);

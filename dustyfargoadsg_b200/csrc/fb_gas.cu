@@ -110,6 +110,7 @@ static __device__ double block_min_dyn(double v, double *sh)
 }
 
 static __device__ void controller_body(const KP &k, double *sh, fb_ctl *c);
+static __device__ __forceinline__ void lost_mass_sum(const KP &k);
 static __device__ void planet_prelude(const KP &k, fb_ctl *c);
 // Work arrays of the planets' step.  k_planets is one thread and keeps them
 // in shared memory: with them as local arrays of the thread, the device
@@ -142,6 +143,36 @@ static inline int cfl_threads(int ns)
   const int t = ((ns + 3) / 4 + 31) / 32 * 32;
   return t < CFL_BS ? t : CFL_BS;
 }
+// The last CTA to finish runs the controller (no waiting: whoever comes last
+// sees every other ring's results).  With has_h it then sets the loop
+// condition h: another substep follows.
+static __device__ __forceinline__ void controller_last_cta(const KP &k, double *sh, cudaGraphConditionalHandle h,
+                                                           int has_h)
+{
+  const int tid = threadIdx.x, T = blockDim.x;
+  __shared__ int last;
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    last = (atomicAdd(&k.ctl->cfl_done, 1u) == gridDim.x - 1) ? 1 : 0;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  __shared__ fb_ctl cs;
+  unsigned long long *dst = (unsigned long long *)&cs;
+  const unsigned long long *src = (const unsigned long long *)k.ctl;
+  for (int w = tid; w < (int)(sizeof(fb_ctl) / 8); w += T) dst[w] = __ldcg(src + w);
+  __syncthreads();
+  controller_body(k, sh, &cs);
+  __syncthreads();
+  if (tid == 0) cs.cfl_done = 0;
+  __syncthreads();
+  unsigned long long *out = (unsigned long long *)k.ctl;
+  for (int w = tid; w < (int)(sizeof(fb_ctl) / 8); w += T) out[w] = dst[w];
+  if (has_h && tid == 0) cudaGraphSetConditional(h, 1);
+}
+
 __global__ void __launch_bounds__(CFL_BS, 4) k_cfl(KP k)
 {
   fb_grid_dependency();
@@ -255,28 +286,7 @@ __global__ void __launch_bounds__(CFL_BS, 4) k_cfl(KP k)
     smax = -block_min_dyn(-smax, sh);
     if (tid == 0) k.ringmin[i] = (smax > 0.0) ? FB_CFLSECURITY / sqrt(smax) : 1e30;
   }
-  // the last CTA to finish runs the controller (no waiting: whoever comes
-  // last sees every other ring's results)
-  __shared__ int last;
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    last = (atomicAdd(&k.ctl->cfl_done, 1u) == gridDim.x - 1) ? 1 : 0;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  __shared__ fb_ctl cs;
-  unsigned long long *dst = (unsigned long long *)&cs;
-  const unsigned long long *src = (const unsigned long long *)k.ctl;
-  for (int w = tid; w < (int)(sizeof(fb_ctl) / 8); w += T) dst[w] = __ldcg(src + w);
-  __syncthreads();
-  controller_body(k, sh, &cs);
-  __syncthreads();
-  if (tid == 0) cs.cfl_done = 0;
-  __syncthreads();
-  unsigned long long *out = (unsigned long long *)k.ctl;
-  for (int w = tid; w < (int)(sizeof(fb_ctl) / 8); w += T) out[w] = dst[w];
+  controller_last_cta(k, sh, 0, 0);
 }
 
 void fb_launch_cfl(const KP &k, cudaStream_t s)
@@ -520,6 +530,7 @@ static __device__ void planet_prelude(const KP &k, fb_ctl *c)
 static __device__ void controller_body(const KP &k, double *sh, fb_ctl *c)
 {
   const int nr = k.nr, tid = threadIdx.x, T = blockDim.x;
+  if (tid == 0) c->go = 1;  // the substep it sets up runs
   // ConditionCFL reduction (SourceEuler.c:1336-1497), the ring partials of
   // the forces and sums; every load is issued before the reductions
   double m = 1e30;
@@ -3086,6 +3097,269 @@ __global__ void __launch_bounds__(FB_BS) k_damping(KP k, double dtov)
 void fb_launch_damping(const KP &k, double dt_override, cudaStream_t s)
 {
   if (k.n_damp_rings > 0) fb_launch(k_damping, k.n_damp_rings, FB_BS, 0, s, k, dt_override);
+}
+
+// ------------------------------------------------------------ end of a substep
+// ComputeVelocities' radial part, floors and walls (k_transport_vr), the
+// Stockholm damping (k_damping), the next substep's ConditionCFL with the
+// controller (k_cfl) and, with fuse_cs, its sound speed (k_soundspeed) in one
+// pass: one
+// CTA per ring, the ring's E cells per thread in registers from the
+// transport's outputs to the time step's limits.  The CFL limits need the
+// radial velocity of the ring above: it is evaluated (and damped, from its own
+// ring mean) here too.  Discs with walls only: the other edges change rings
+// between these steps.  The last substep of a DT (done, set by its own
+// controller) has no successor: its CTAs stop after the damping and the loop
+// ends.
+struct FinRing {  // the damping of one ring: the targets, lambda, and the shared reciprocal of 1 + lambda
+  double lam, den, rden;
+  bool on, zero;
+};
+static __device__ __forceinline__ FinRing fin_ring(const KP &k, int i, double step)
+{
+  FinRing f = {0.0, 1.0, 1.0, false, false};
+  if (!k.evanescent || i >= k.nr) return f;
+  const double r = k.rmed[i];
+  const bool lo = r < k.wkzrmin, hi = r > k.wkzrmax;
+  if (!lo && !hi) return f;
+  f.on = true;
+  f.lam = k.damp_lam[i] * step / k.damp_tau[i];
+  f.den = 1.0 + f.lam;
+  f.rden = 1.0 / f.den;
+  f.zero = k.zero_vrad && ((lo && (i == 0 || i == 1)) || (hi && i == k.nr - 1));
+  return f;
+}
+
+template <int E, bool ENERGY, int MT>
+__global__ void __launch_bounds__(MT, 2) k_finish(KP k, int fuse_cs, cudaGraphConditionalHandle h, int has_h)
+{
+  fb_grid_dependency();
+  __shared__ double sh[7 * 32];
+  extern __shared__ double fin_vt[];  // the ring's final vtheta
+  const int i = blockIdx.x, ns = k.ns, nr = k.nr, T = blockDim.x, tid = threadIdx.x;
+  const size_t base = (size_t)i * ns;
+  const double step = k.ctl->dt;
+  const bool stop = k.ctl->done || k.ctl->status;  // no substep follows
+  const bool capped = k.ctl->substeps >= k.cap;
+  const bool cfl = !stop && !capped;
+  const int wall = k.wall;
+  // every load first: the cell's density, the momenta of the faces at its
+  // ring and the ring above, vtheta, energy, sound speed
+  double d[E], v[E], vp[E], vt[E], en[E], cs[E];
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    const int j = tid + e * T;
+    d[e] = v[e] = vp[e] = vt[e] = en[e] = cs[e] = 0.0;
+    if (j >= ns) continue;
+    // ComputeVelocities (TransportEuler.c:531-536) at interface ring ii
+    auto vr_at = [&](int ii) -> double {
+      if (ii == 0) return 0.0;
+      const size_t m = (size_t)ii * ns + j;
+      return (k.q[0][m - ns] + k.q[1][m]) / (k.rho_t[m] + k.rho_t[m - ns] + 1e-20);
+    };
+    d[e] = k.rho_t[base + j];
+    vt[e] = k.vt[base + j];
+    if (ENERGY) en[e] = k.e[base + j];
+    if (cfl) cs[e] = k.cs[base + j];
+    const int src = !wall ? i : i == 0 ? -2 : (i == 1 || i == nr - 1) ? 0 : i;
+    v[e] = (src < 0) ? -vr_at(-src) : vr_at(src);
+    if (cfl || i == nr - 1) {  // the ring above (ring nr: the outer wall's mirror)
+      const int up = i + 1;
+      const int srcp = up == nr ? (wall ? -(nr - 2) : 0) : !wall ? up : (up == 1 || up == nr - 1) ? 0 : up;
+      vp[e] = (srcp < 0) ? -vr_at(-srcp) : vr_at(srcp);
+    }
+    if (k.add_floors && d[e] < k.floordens) d[e] = k.floordens;
+    if (wall && (i <= 1 || i >= nr - 2)) d[e] = k.sigmamed[i];
+  }
+  if (i == 0 && tid == 0 && cfl) planet_prelude(k, k.ctl);
+  if (i == ((nr > 2) ? 2 : 0) && (tid >> 5) == 0) lost_mass_sum(k);  // by a ring off the planets' path
+  // ---- EvanescentBoundary (SideEuler.c:796-950)
+  const FinRing f = fin_ring(k, i, step), fp = fin_ring(k, cfl ? i + 1 : nr, step);
+  if (f.on || fp.on) {
+    double vrad0, vradp0, vtheta0, dens0, energ0;
+    if (k.damp_axi) {
+      double m[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int e = 0; e < E; e++) {  // cells past the ring are zero
+        m[0] += v[e];
+        m[1] += vt[e];
+        if (tid + e * T < ns) m[2] += d[e];
+        m[3] += en[e];
+        m[4] += vp[e];
+      }
+      block_sums<5>(m, sh);
+      vrad0 = m[0] / (double)ns;
+      vtheta0 = m[1] / (double)ns;
+      dens0 = m[2] / (double)ns;
+      energ0 = m[3] / (double)ns;
+      vradp0 = m[4] / (double)ns;
+    } else {
+      vtheta0 = k.vthetamed[i] - k.rmed[i] * omf(k);
+      vrad0 = k.vradmed[i];
+      vradp0 = fp.on ? k.vradmed[i + 1] : 0.0;
+      dens0 = k.sigmamed[i];
+      energ0 = k.energymed[i];
+    }
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      if (f.on) {
+        v[e] = f.zero ? 0.0 : fb_quot(v[e] + f.lam * vrad0, f.den, f.rden);
+        d[e] = f.zero ? dens0 : fb_quot(d[e] + f.lam * dens0, f.den, f.rden);
+        vt[e] = f.zero ? vtheta0 : fb_quot(vt[e] + f.lam * vtheta0, f.den, f.rden);
+        if (ENERGY) en[e] = fb_quot(en[e] + f.lam * energ0, f.den, f.rden);
+      }
+      if (fp.on) vp[e] = fp.zero ? 0.0 : fb_quot(vp[e] + fp.lam * vradp0, fp.den, fp.rden);
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    const int j = tid + e * T;
+    if (j >= ns) continue;
+    k.rho[base + j] = d[e];
+    k.vr[base + j] = v[e];
+    if (i == nr - 1 && wall) k.vr[base + ns + j] = vp[e];
+    if (f.on) {
+      k.vt[base + j] = vt[e];
+      if (ENERGY) k.e[base + j] = en[e];
+    }
+    if (cfl) fin_vt[j] = vt[e];
+  }
+  if (!cfl) {
+    if (i == 0 && tid == 0) {
+      if (!stop) k.ctl->status = FB_ERR_SUBSTEPS;  // the cap bounds the loop even if the time step collapses
+      k.ctl->go = 0;
+      if (has_h) cudaGraphSetConditional(h, 0);
+    }
+    return;
+  }
+  __syncthreads();
+  // ---- ConditionCFL, ring sums and DetectCrash: see k_cfl
+  const double rmi = k.rmed[i], surf = k.surf[i], rs = k.indirect_smoothing;
+#if FB_FAST
+  const double dist2_ring = rmi * rmi + rs * rs;
+  const double invd3_ring = 1.0 / dist2_ring / sqrt(dist2_ring);
+#endif
+  double s[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  const double dxrad = k.dxrad[i], dxtheta = k.dxtheta_cfl[i];
+  const double dxmin = min2(dxrad, dxtheta);
+  const double rdxmin = 1.0 / dxmin, rdxrad = 1.0 / dxrad, rdxtheta = 1.0 / dxtheta;
+  int negd = 0, nege = 0, bad = 0;
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    const int j = tid + e * T;
+    if (j >= ns) continue;
+    s[0] += vt[e];
+    if (d[e] < 0.0) negd = 1;
+    if (!isfinite(d[e]) || !isfinite(vt[e]) || !isfinite(v[e])) bad = 1;
+    if (ENERGY) {
+      if (en[e] < 0.0) nege = 1;
+      if (!isfinite(en[e])) bad = 1;
+    }
+    const double xc = rmi * k.cosaz[j];
+    const double yc = rmi * k.sinaz[j];
+    const double cellmass = surf * d[e];
+#if FB_FAST
+    const double InvDist3 = invd3_ring;
+#else
+    const double dist2 = xc * xc + yc * yc + rs * rs;
+    const double distance = sqrt(dist2);
+    const double InvDist3 = 1.0 / dist2 / distance;
+#endif
+    s[1] += FB_G * cellmass * xc * InvDist3 * 1.0;
+    s[2] += FB_G * cellmass * yc * InvDist3 * 1.0;
+    s[3] += cellmass;
+    s[4] += cellmass * xc;
+    s[5] += cellmass * yc;
+    double csn = 0.0;
+    if (ENERGY && fuse_cs) {  // ComputeSoundSpeed of the new state (SourceEuler.c:2323-2343), after this limit's use of the old
+      csn = sqrt(k.gamma * (k.gamma - 1.0) * en[e] / d[e]);
+      s[6] += csn;
+    }
+    const int jp = (j == ns - 1) ? 0 : j + 1;
+    const double invdt1 = fb_quot(cs[e], dxmin, rdxmin);
+    const double invdt2 = fb_quot(fabs(v[e]), dxrad, rdxrad);
+    double dvr = vp[e] - v[e];
+    double dvt = fin_vt[jp] - vt[e];
+    if (dvr >= 0.0) dvr = 1e-10; else dvr = -dvr;
+    if (dvt >= 0.0) dvt = 1e-10; else dvt = -dvt;
+    double invdt4 = max2(fb_quot(dvr, dxrad, rdxrad), fb_quot(dvt, dxtheta, rdxtheta));
+    invdt4 *= 4.0 * FB_CVNR * FB_CVNR;
+    if (ENERGY && fuse_cs) k.cs[base + j] = csn;
+    v[e] = invdt1 * invdt1 + invdt2 * invdt2;  // the sum under the root, in parts
+    vp[e] = invdt4 * invdt4;
+  }
+  block_sums<7>(s, sh);
+  const double vmoy = s[0] / (double)ns;
+  if (tid == 0) {
+    k.vmoy[i] = vmoy;
+    double *pp = k.partials + (size_t)i * 5;  // summed by the controller in ring order
+    for (int q = 0; q < 5; q++) pp[q] = s[1 + q];
+  }
+  const int flags = __syncthreads_or(negd | (nege << 1) | (bad << 2));
+  if (tid == 0) {
+    if (flags & 1) atomicOr(&k.ctl->neg_dens_flag, 1);
+    if (flags & 2) atomicOr(&k.ctl->neg_energy_flag, 1);
+    if (flags & 4) atomicOr(&k.ctl->nonfinite, 1);
+  }
+  if (i >= 1) {
+    const double viscosity = nu_ring(k, i);
+    const double invdt5 = (viscosity != 0.0) ? viscosity * 4.0 / k.mindx2[i] : 1e-10;
+    const double invdt6 = (ENERGY && k.ent_diff) ? k.diffusivity * 4.0 / k.mindx2[i] : 1e-10;
+    double smax = -1.0;
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+      if (tid + e * T >= ns) continue;
+      const double vres = k.fast_transport ? vt[e] - vmoy : vt[e];
+      const double invdt3 = fb_quot(fabs(vres), dxtheta, rdxtheta);
+      const double S = v[e] + invdt3 * invdt3 + vp[e] + invdt5 * invdt5 + invdt6 * invdt6;
+      if (S > smax) smax = S;
+    }
+    smax = -block_min_dyn(-smax, sh);
+    if (tid == 0) k.ringmin[i] = (smax > 0.0) ? FB_CFLSECURITY / sqrt(smax) : 1e30;
+  }
+  if (ENERGY && fuse_cs && k.visc_mode == 1) {
+    __syncthreads();  // nu_ring's reads of the old mean
+    if (tid == 0) k.gcs[i] = s[6] / (double)ns;
+  }
+  controller_last_cta(k, sh, h, has_h);
+}
+
+// Where the end of the substep is one launch of k_finish: while all rings' CTAs
+// are on the GPU at once.  There the substep is bound by its chain of launches
+// and one of them does the work of three or four (us per substep, with
+// k_transport_vr, k_damping, k_cfl and k_soundspeed against k_finish: 48 x 144
+// 41.9 / 35, 128 x 384 47.3 / 38, 256 x 768 with particles 112 / 106).  On
+// larger grids a CTA's own chain of reductions is what a wave waits for, and
+// the per-cell kernels fill the GPU better (333 x 1001 adiabatic 108 / 114,
+// 768 x 2304 247 / 287).
+int fb_finish_fits(const KP &k)
+{
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 0;
+  return k.nr <= 2 * sms && k.ns <= 1024;
+}
+
+// One cell per thread up to 384 azimuths, else two (128 x 384: 18.1 us a stage
+// with one, 22.0 with four; 256 x 768: 22.0 with two, 28.6 with one).
+template <bool ENERGY>
+static void launch_finish(const KP &k, int fuse_cs, cudaGraphConditionalHandle h, int has_h, cudaStream_t s)
+{
+  const size_t sm = (size_t)k.ns * sizeof(double);
+  auto T = [&](int E) { return ((k.ns + E - 1) / E + 31) / 32 * 32; };
+  if (k.ns <= 384)
+    fb_launch(k_finish<1, ENERGY, 384>, k.nr, T(1), sm, s, k, fuse_cs, h, has_h);
+  else
+    fb_launch(k_finish<2, ENERGY, 512>, k.nr, T(2), sm, s, k, fuse_cs, h, has_h);
+}
+
+void fb_launch_finish(const KP &k, int fuse_cs, const cudaGraphConditionalHandle *h, cudaStream_t s)
+{
+  const cudaGraphConditionalHandle hh = h ? *h : 0;
+  if (k.energy)
+    launch_finish<true>(k, fuse_cs, hh, h ? 1 : 0, s);
+  else
+    launch_finish<false>(k, fuse_cs, hh, h ? 1 : 0, s);
 }
 
 // ------------------------------------------------------------ diagnostics
