@@ -1531,10 +1531,9 @@ extern "C" int fb_get_tuning(const fb_ctx *ctx, fb_tuning *t)
   if (!ctx || !t) return FB_ERR_INVALID;
   const KP &k = ctx->k;
   t->cell_block = k.cell_bs;
-  t->azi_cells_per_thread = k.azi_E > 0 ? k.azi_E : fb_azi_E_auto(k.ns);
   t->rad_columns = k.rad_tx > 0 ? k.rad_tx : 64;
   t->rad_rings = k.rad_chunk > 0 ? k.rad_chunk : fb_rad_chunk_auto(k);
-  t->azi_variant = fb_azi_variant(k.ns, k.energy, t->azi_cells_per_thread, k.azi_variant);
+  t->azi_variant = fb_azi_shape(k, &t->azi_cells_per_thread);
   return FB_OK;
 }
 

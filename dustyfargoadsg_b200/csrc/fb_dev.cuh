@@ -402,6 +402,7 @@ int  fb_transport_preload(void);          // loads the radial and vr transport k
 int  fb_azi_E_valid(int ns, int energy, int E);   // 1 if E cells/thread fit this ring
 int  fb_azi_E_auto(int ns);
 int  fb_azi_launches(const KP &k);  // kernel launches of one azimuthal pass
+int  fb_azi_shape(const KP &k, int *E);  // the variant and cells per thread in effect
 int  fb_azi_variant(int ns, int energy, int E, int variant);  // variant a launch takes (0: cannot run)
 int  fb_rad_chunk_auto(const KP &k);
 int  fb_rad_chunks_balanced(const KP &k, int tx, int *out, int max);

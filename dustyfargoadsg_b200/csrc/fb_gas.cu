@@ -2419,9 +2419,26 @@ int fb_azi_variant(int ns, int energy, int E, int variant)
 // The variant and cells per thread a launch of this KP's azimuthal pass
 // takes: the tuned ones where they can run, the staged variant only on
 // 16-byte aligned fields, the tile variant only with its scratch fields.
+//
+// Not tuned: the tile variant with two cells per lane (three for rings that
+// need them) from FB_AZT_MIN_CELLS cells on, the fastest or within 2% of it on
+// every grid and both builds measured, 64 x 192 to 700 x 2300 (us per substep,
+// packed / tile, isothermal fast build: 128 x 384 38.5 / 36.4, 192 x 576 49.0 /
+// 43.3, 333 x 1001 88.2 / 71.4, 700 x 2300 325.7 / 233.8; parity build 40.6 /
+// 39.6, 53.4 / 48.2, 96.1 / 81.9, 425.7 / 292.9).  On smaller grids the ring
+// means' own launch costs what the pass gains (32 x 96: 38.0 / 38.9).
+#define FB_AZT_MIN_CELLS 10000
 static int azi_resolve(const KP &k, int *Eout)
 {
   const int NQ = k.energy ? 6 : 5;
+  if (k.azi_E == 0 && k.azi_variant == 0 && k.azt_buf[0] && k.azt_buf[1] && k.azt_buf[2] && k.azt_vmed &&
+      (long)k.nr * k.ns >= FB_AZT_MIN_CELLS) {
+    const int Et = azt_fits(k.ns, 2) ? 2 : 3;
+    if (azt_fits(k.ns, Et)) {
+      if (Eout) *Eout = Et;
+      return 6;
+    }
+  }
   const int E = k.azi_E > 0 ? k.azi_E : fb_azi_E_auto(k.ns);
   int var = fb_azi_variant(k.ns, k.energy, E, k.azi_variant);
   if (var == 0) var = 1;
@@ -2431,6 +2448,7 @@ static int azi_resolve(const KP &k, int *Eout)
   if (Eout) *Eout = E;
   return var;
 }
+int fb_azi_shape(const KP &k, int *E) { return azi_resolve(k, E); }
 static bool azt_variant(int var) { return var == 6 || var == 7 || var == 8; }
 int fb_azi_launches(const KP &k) { return azt_variant(azi_resolve(k, nullptr)) ? 2 : 1; }
 
