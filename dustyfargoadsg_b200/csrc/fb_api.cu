@@ -30,6 +30,8 @@ struct fb_ctx {
   cudaEvent_t ev_fork, ev_planets;    // its start and end within a substep
   cudaStream_t st_sg;                 // branch of the self-gravity convolution
   cudaEvent_t ev_sg_fork, ev_sg_done;
+  cudaStream_t st_dust, st_rng;        // branches of the particles and their candidate pairs
+  cudaEvent_t ev_dust_rng, ev_dust_upd, ev_dust_end;
   cudaEvent_t ev_vm_fork, ev_vm_done;  // the tile variant's ring means, on the SG stream beside SubStep3 / radial
   KP k;
   std::vector<void *> allocs;
@@ -152,9 +154,9 @@ static int dust_create(fb_ctx *ctx)
     set_err(ctx, "particles need a non-rotating frame (OMEGAFRAME = 0)");
     return FB_ERR_UNSUPPORTED;
   }
-  double **grids[] = {&k.indpot, &k.rgp, &k.agp, &k.rind, &k.aind, &k.rsga, &k.asga};
+  double **grids[] = {&k.indpot, &k.rsga, &k.asga, &k.rgp, &k.agp, &k.rind, &k.aind};
   for (size_t f = 0; f < sizeof grids / sizeof grids[0]; f++)
-    if (!(*grids[f] = dalloc(ctx, nf))) return FB_ERR_NOMEM;
+    if (!(*grids[f] = dalloc(ctx, f < 3 ? nf : 2 * nf))) return FB_ERR_NOMEM;
   k.particles = 1;
   k.dust_feel_planets = p->dust_feel_planets;
   k.dust_feel_disk = p->dust_feel_disk;
@@ -274,7 +276,12 @@ extern "C" int fb_create(const fb_params *p, const double *radii, fb_ctx **out)
       cudaEventCreateWithFlags(&ctx->ev_sg_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_sg_done, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_vm_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&ctx->ev_vm_done, cudaEventDisableTiming) != cudaSuccess) {
+      cudaEventCreateWithFlags(&ctx->ev_vm_done, cudaEventDisableTiming) != cudaSuccess ||
+      (p->nbpart > 0 && (cudaStreamCreateWithFlags(&ctx->st_dust, cudaStreamNonBlocking) != cudaSuccess ||
+                         cudaStreamCreateWithFlags(&ctx->st_rng, cudaStreamNonBlocking) != cudaSuccess ||
+                         cudaEventCreateWithFlags(&ctx->ev_dust_rng, cudaEventDisableTiming) != cudaSuccess ||
+                         cudaEventCreateWithFlags(&ctx->ev_dust_upd, cudaEventDisableTiming) != cudaSuccess ||
+                         cudaEventCreateWithFlags(&ctx->ev_dust_end, cudaEventDisableTiming) != cudaSuccess))) {
     fb_destroy(ctx);
     return FB_ERR_CUDA;
   }
@@ -587,6 +594,11 @@ extern "C" int fb_destroy(fb_ctx *ctx)
   if (ctx->ev_vm_fork) cudaEventDestroy(ctx->ev_vm_fork);
   if (ctx->ev_vm_done) cudaEventDestroy(ctx->ev_vm_done);
   if (ctx->st_sg) cudaStreamDestroy(ctx->st_sg);
+  if (ctx->ev_dust_rng) cudaEventDestroy(ctx->ev_dust_rng);
+  if (ctx->ev_dust_upd) cudaEventDestroy(ctx->ev_dust_upd);
+  if (ctx->ev_dust_end) cudaEventDestroy(ctx->ev_dust_end);
+  if (ctx->st_dust) cudaStreamDestroy(ctx->st_dust);
+  if (ctx->st_rng) cudaStreamDestroy(ctx->st_rng);
   for (auto &e : ctx->pev) cudaEventDestroy(e);
   if (ctx->gdt_exec) cudaGraphExecDestroy(ctx->gdt_exec);
   if (ctx->gdt) cudaGraphDestroy(ctx->gdt);
@@ -772,8 +784,22 @@ static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NU
   }
   // particles after the planets' RK5 step and before the gas update
   // (SourceEuler.c:504-531)
-  if (ctx->has_dust)
-    STAGE(ST_DUST, fb_dust_launches(ctx->pp), fb_launch_dust_substep(k, ctx->pp, s, ctx->ev_planets));
+  // The isothermal gas kernels up to the azimuthal transport leave alone what
+  // the particles read (the state, and the half of the gradient grids the
+  // previous substep wrote), so the particles run beside them; with the energy
+  // equation the sound speed they read changes before that, and the
+  // self-gravity kicks write the grids they read: in line there.
+  const bool dust_branch = ctx->has_dust && !ctx->profiling && !k.energy && !k.self_gravity;
+  if (dust_branch) {
+    cudaStreamWaitEvent(ctx->st_dust, ctx->ev_fork, 0);
+    fb_launch_dust_substep(k, ctx->pp, ctx->st_dust, ctx->st_rng, ctx->ev_fork, ctx->ev_dust_rng, ctx->ev_planets,
+                           ctx->ev_dust_upd);
+    cudaEventRecord(ctx->ev_dust_end, ctx->st_dust);
+    ctx->launches += fb_dust_launches(ctx->pp);
+    ctx->pcount[ST_DUST] += fb_dust_launches(ctx->pp);
+  } else if (ctx->has_dust) {
+    STAGE(ST_DUST, fb_dust_launches(ctx->pp), fb_launch_dust_substep(k, ctx->pp, s, s, NULL, NULL, ctx->ev_planets, NULL));
+  }
   // SubStep0: thermal diffusion, before the sound speed (SourceEuler.c:577-586)
   if (k.energy && (k.ent_diff || k.rad_diff)) {
     int n0 = 0;  // the stage's kernel launches
@@ -813,6 +839,7 @@ static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NU
   }
   if (k.energy) STAGE(ST_SUB3, 1, fb_launch_substep3(k, s));  // with the stresses of the new velocities
   STAGE(ST_TRAD, 1, fb_launch_transport_radial(kt, 0.0, s));
+  if (dust_branch) cudaStreamWaitEvent(s, ctx->ev_dust_upd, 0);  // the azimuthal pass writes vtheta
   if (vm_branch) {
     cudaStreamWaitEvent(s, ctx->ev_vm_done, 0);
     STAGE(ST_TAZI, 1, fb_launch_transport_azimuthal(kt, 0.0, s, true));
@@ -832,6 +859,7 @@ static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NU
   }
   if (!at_end && k.evanescent && k.n_damp_rings > 0) STAGE(ST_DAMP, 1, fb_launch_damping(k, 0.0, s));
   if (!ctx->has_dust) cudaStreamWaitEvent(s, ctx->ev_planets, 0);
+  if (dust_branch) cudaStreamWaitEvent(s, ctx->ev_dust_end, 0);
   if (at_end) {
     STAGE(ST_FIN, 1, fb_launch_finish(k, cs_done, h, s));
   } else if (h) {
@@ -1574,8 +1602,9 @@ static int snapshot_take(fb_ctx *ctx, Snapshot &sn)
   if (ctx->has_dust) {
     PP &pp = ctx->pp;
     const size_t np = (size_t)pp.n * sizeof(double);
-    double *g[] = {k.indpot, k.rgp, k.agp, k.rind, k.aind, k.rsga, k.asga};
+    double *g[] = {k.indpot, k.rsga, k.asga}, *g2[] = {k.rgp, k.agp, k.rind, k.aind};
     for (double *f : g) sn.regions.push_back({f, nf});
+    for (double *f : g2) sn.regions.push_back({f, 2 * nf});
     double *a[] = {pp.r, pp.th, pp.vr, pp.vth, pp.l, pp.size, pp.st};  // permuted by the DT's sort
     for (double *f : a) sn.regions.push_back({f, np});
     sn.regions.push_back({pp.orig, (size_t)pp.n * sizeof(int)});

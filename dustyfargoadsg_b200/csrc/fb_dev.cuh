@@ -24,6 +24,7 @@ struct fb_ctl {
   double bary_x[3], bary_y[3];               // stardiscbarycenter_{x,y}
   double mdisc;
   int substeps, done, status, nonfinite;
+  int flip;               // which half of the particles' gradient grids this substep writes (dust_grid_write)
   int go;                 // the loop runs another substep (k_finish; else it goes on while not done)
   // DetectCrash (SourceEuler.c:51-69) as AlgoGas uses it (:545-566): the
   // CFL kernel's CTAs raise the flags for the state at the start of the
@@ -165,7 +166,10 @@ struct KP {
   int transport_only;      // stage test: Transport without floors/boundaries
   // Lagrangian particles: grids the gas substep leaves for the next particle
   // update (IndPotential, RadGradP, AziGradP, RadIndAcc, AziIndAcc,
-  // RadSGAcc, AziSGAcc of src/SourceEuler.c:210-216); NULL without particles
+  // RadSGAcc, AziSGAcc of src/SourceEuler.c:210-216); NULL without particles.
+  // RadGradP, AziGradP, RadIndAcc and AziIndAcc have two halves of nf values, by
+  // turns: a substep's gas kernels write one while its particles read the
+  // other, the previous substep's
   double *indpot, *rgp, *agp, *rind, *aind, *rsga, *asga;
   int particles, dust_feel_planets, dust_feel_disk;
   // DUSTFEEDBACK: the substep is also bounded by half the particles' minimum
@@ -203,6 +207,9 @@ struct KP {
 // OmegaFrame as the current substep sees it: the control block's in a
 // corotating frame (updated by the planets' step), else the constant
 static __device__ __forceinline__ double omf(const KP &k) { return k.corot ? k.ctl->omega_frame : k.omega_frame; }
+
+static __device__ __forceinline__ size_t dust_grid_write(const KP &k) { return k.ctl->flip ? k.nf : 0; }
+static __device__ __forceinline__ size_t dust_grid_read(const KP &k) { return k.ctl->flip ? 0 : k.nf; }
 
 // Device state of the particles' random stream (src/DustUpdate.c:438-485).
 // a / d rounded to nearest, given r = 1/d rounded to nearest (fb_rcp in the
@@ -427,7 +434,10 @@ void fb_launch_body_force(const KP &k, double x, double y, double rsmoothing, do
                           cudaStream_t s);
 void fb_launch_ring_mean(const double *f, int nr, int ns, double *out, cudaStream_t s);
 // Lagrangian particles (fb_dust.cu)
-void fb_launch_dust_substep(const KP &k, const PP &pp, cudaStream_t s, cudaEvent_t planets_done);
+// s: the particles' chain; srng: the candidate pairs (may be s); the update
+// waits for planets_done, and updated (if any) marks its end
+void fb_launch_dust_substep(const KP &k, const PP &pp, cudaStream_t s, cudaStream_t srng, cudaEvent_t fork,
+                            cudaEvent_t rng_done, cudaEvent_t planets_done, cudaEvent_t updated);
 void fb_launch_dust_interpolation_only(const KP &k, const PP &pp, cudaStream_t s);
 int  fb_dust_launches(const PP &pp);
 int fb_launch_dust_sort(const KP &k, const PP &pp, cudaStream_t s);  // returns launches

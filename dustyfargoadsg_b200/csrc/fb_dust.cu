@@ -275,14 +275,16 @@ static __device__ __forceinline__ long long candidate_limit(const PP &pp, int np
   return lim < pp.ncand ? lim : pp.ncand;
 }
 
+// The acceptance of every candidate a substep can need: it depends on the
+// stream's position alone, so it runs beside the drift and the ranking that
+// find how many are needed.
 __global__ void __launch_bounds__(D_BS) k_rng_count(PP pp)
 {
   fb_grid_dependency();
   __shared__ int sh[D_BS / 32];
   const long long c = (long long)blockIdx.x * D_BS + threadIdx.x;
-  const int npairs = pp.dc->npairs;
   int acc = 0;
-  if (npairs > 0 && c < candidate_limit(pp, npairs)) {
+  if (c < pp.ncand) {
     double u1, u2, w;
     acc = candidate(pp.dc->x, c, &u1, &u2, &w) ? 1 : 0;
   }
@@ -298,9 +300,8 @@ __global__ void __launch_bounds__(D_BS) k_rng_count(PP pp)
 }
 
 // Accepted candidate number g (in stream order) becomes pair g.  The
-// blocks' counts are summed here: only the blocks below the candidate limit
-// have any (a handful), and each of those adds the counts before it; block 0
-// also checks that the candidates cover the pairs needed -- never silently
+// blocks' counts are summed here: each block that holds a needed candidate adds
+// the counts before it; block 0 also checks that the candidates cover the pairs needed -- never silently
 // wrong: the step stops with an error status.
 __global__ void __launch_bounds__(D_BS) k_rng_scatter(KP k, PP pp, int nb)
 {
@@ -322,7 +323,8 @@ __global__ void __launch_bounds__(D_BS) k_rng_scatter(KP k, PP pp, int nb)
     return t;
   };
   if (blockIdx.x == 0) {
-    const int total = block_count(nb);
+    const long long lim = candidate_limit(pp, npairs);
+    const int total = block_count((int)((lim + D_BS - 1) / D_BS < nb ? (lim + D_BS - 1) / D_BS : nb));
     if (threadIdx.x == 0 && npairs > total) {
       pp.dc->err = 1;
       k.ctl->status = FB_ERR_INVALID;
@@ -482,6 +484,7 @@ __global__ void __launch_bounds__(D_BS, 3) k_dust_update(KP k, PP pp, int mode)
       wt_i[t] = tsc_weight(fabs(tp - az), delta_phi, rdelta_phi);
     }
   }
+  const size_t dgrid = dust_grid_read(k);
   // ---- 2a) vrad-staggered values: (Rinf[i], Azimuth[j]) (Dsys.c:397-487)
 #pragma unroll
   for (int tj = 0; tj < 3; tj++) {
@@ -493,8 +496,8 @@ __global__ void __launch_bounds__(D_BS, 3) k_dust_update(KP k, PP pp, int mode)
       const double wr = wr_inf[ti];
       const size_t l = (size_t)i * ns + jc[tj];
       vrg += (wr * wt * k.vr[l]);
-      rgp += (wr * wt * k.rgp[l]);
-      if (k.indirect_term) rind += (wr * wt * k.rind[l]);
+      rgp += (wr * wt * k.rgp[l + dgrid]);
+      if (k.indirect_term) rind += (wr * wt * k.rind[l + dgrid]);
       if (want_sg) rsg += (wr * wt * k.rsga[l]);
     }
   }
@@ -511,8 +514,8 @@ __global__ void __launch_bounds__(D_BS, 3) k_dust_update(KP k, PP pp, int mode)
       const double wr = wr_med[ti];
       const size_t l = (size_t)i * ns + ji[tj];
       vtg += (wr * wt * k.vt[l]);
-      agp += (wr * wt * k.agp[l]);
-      if (k.indirect_term) aind += (wr * wt * k.aind[l]);
+      agp += (wr * wt * k.agp[l + dgrid]);
+      if (k.indirect_term) aind += (wr * wt * k.aind[l + dgrid]);
       if (want_sg) asg += (wr * wt * k.asga[l]);
     }
   }
@@ -739,20 +742,30 @@ void fb_launch_dust_to_reference_order(const PP &pp, const double *src, double *
 // ---------------------------------------------------------- launchers
 int fb_dust_launches(const PP &pp) { return pp.feel_turb ? 7 : 2; }
 
-void fb_launch_dust_substep(const KP &k, const PP &pp, cudaStream_t s, cudaEvent_t planets_done)
+void fb_launch_dust_substep(const KP &k, const PP &pp, cudaStream_t s, cudaStream_t srng, cudaEvent_t fork,
+                            cudaEvent_t rng_done, cudaEvent_t planets_done, cudaEvent_t updated)
 {
   const int nb = (pp.n + D_BS - 1) / D_BS;
+  const int ncb = (pp.ncand + D_BS - 1) / D_BS;
+  if (pp.feel_turb && srng != s) {
+    cudaStreamWaitEvent(srng, fork, 0);
+    fb_launch(k_rng_count, ncb, D_BS, 0, srng, pp);
+    cudaEventRecord(rng_done, srng);
+  }
   fb_launch(k_dust_drift, nb, D_BS, 0, s, k, pp);
   if (pp.feel_turb) {
     const int nsb = (pp.n + SCAN_BS - 1) / SCAN_BS;
     fb_launch(k_scan_block, nsb, SCAN_BS, 0, s, pp.flag, pp.kidx, pp.kick_bsum, pp.n);
     fb_launch(k_kick_top, 1, SCAN_BS, 0, s, pp, nsb);
-    const int ncb = (pp.ncand + D_BS - 1) / D_BS;
-    fb_launch(k_rng_count, ncb, D_BS, 0, s, pp);
+    if (srng != s)
+      cudaStreamWaitEvent(s, rng_done, 0);
+    else
+      fb_launch(k_rng_count, ncb, D_BS, 0, s, pp);
     fb_launch(k_rng_scatter, ncb, D_BS, 0, s, k, pp, ncb);
   }
   if (planets_done) cudaStreamWaitEvent(s, planets_done, 0);  // positions after the planets' step
   fb_launch(k_dust_update, nb, D_BS, 0, s, k, pp, 0);
+  if (updated) cudaEventRecord(updated, s);
   if (pp.feel_turb) fb_launch(k_dust_finish, 1, 1, 0, s, pp);
 }
 

@@ -586,6 +586,7 @@ static __device__ void controller_body(const KP &k, double *sh, fb_ctl *c)
     return;
   }
   const int gastimestepcfl = (int)ncfl;
+  c->flip ^= 1;
   const double dthydro = (c->DT - c->dtemp) / (double)gastimestepcfl;
   const double dt = min2(dthydro, dtnbody);
   c->dthydro = dthydro;
@@ -763,6 +764,7 @@ __global__ void __launch_bounds__(FB_BS2, 4) k_substep1(KP k)
     ipjm = k.indpot[ljm];
     if (i >= 1) iplim = k.indpot[lim];
   }
+  const size_t lg = l + dust_grid_write(k);
   if (keep) k.pres[l] = Pl;  // nothing but fb_download_derived reads it
   if (i >= 1) {
     double gradp = (Pl - Plim) * 2.0 / (rl + rlim) * invdiffrmed;
@@ -772,8 +774,8 @@ __global__ void __launch_bounds__(FB_BS2, 4) k_substep1(KP k)
     vt2 = vt2 * vt2;
     k.vri[l] = vrl + dt * (-gradp - gradphi + vt2 * invrinf);
     if (k.particles) {  // RadGradP, RadIndAcc (SourceEuler.c:875-877)
-      k.rgp[l] = (Pl - Plim) * invdiffrmed;
-      k.rind[l] = -(ipl - iplim) * invdiffrmed;
+      k.rgp[lg] = (Pl - Plim) * invdiffrmed;
+      k.rind[lg] = -(ipl - iplim) * invdiffrmed;
     }
   }
   {
@@ -783,8 +785,8 @@ __global__ void __launch_bounds__(FB_BS2, 4) k_substep1(KP k)
     vti += dt * torque;
     k.vti[l] = vti;
     if (k.particles) {  // AziGradP, AziIndAcc (SourceEuler.c:944-951)
-      k.agp[l] = (Pl - Pjm) * invdxtheta;
-      k.aind[l] = -(ipl - ipjm) * invdxtheta;
+      k.agp[lg] = (Pl - Pjm) * invdxtheta;
+      k.aind[lg] = -(ipl - ipjm) * invdxtheta;
     }
   }
 }

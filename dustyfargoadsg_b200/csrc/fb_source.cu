@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(SRC_MAXW * 32, 2) k_sources(KP k, int ntiles)
   const bool keep = c->done || c->status || c->substeps >= k.cap;
   const bool snap = !SG && c->crash_snap_now;  // the first crash's state (WriteDiskPolar ..., 999)
   const bool visc = (k.visc_mode != 0);
+  const size_t dgrid = PART ? dust_grid_write(k) : 0;
   {
     const int np = SG ? 0 : c->np;
     if ((int)threadIdx.x < np) {
@@ -268,8 +269,8 @@ __global__ void __launch_bounds__(SRC_MAXW * 32, 2) k_sources(KP k, int ntiles)
           vt2 = vt2 * vt2;
           vri[q] = vr[q] + dt * (-gradp - gradphi + vt2 * T[T_INVRINF]);
           if (mine) {  // RadGradP, RadIndAcc (SourceEuler.c:875-877)
-            k.rgp[l] = (P[q] - Pb) * idrm;
-            k.rind[l] = -(ip[q] - ipb) * idrm;
+            k.rgp[l + dgrid] = (P[q] - Pb) * idrm;
+            k.rind[l + dgrid] = -(ip[q] - ipb) * idrm;
           }
         }
         const double idx = T[T_INVDXTHETA];
@@ -278,8 +279,8 @@ __global__ void __launch_bounds__(SRC_MAXW * 32, 2) k_sources(KP k, int ntiles)
         vti[q] = vt[q] - dt * (gradp + gradphi);
         vti[q] += dt * T[T_TORQUE];
         if (mine) {  // AziGradP, AziIndAcc (SourceEuler.c:944-951)
-          k.agp[l] = (P[q] - Pm) * idx;
-          k.aind[l] = -(ip[q] - ipm) * idx;
+          k.agp[l + dgrid] = (P[q] - Pm) * idx;
+          k.aind[l + dgrid] = -(ip[q] - ipm) * idx;
         }
       }
     }
