@@ -367,6 +367,25 @@ extern "C" int fb_create(const fb_params *p, const double *radii, fb_ctx **out)
   k.vradmed = dalloc(ctx, nr);
   k.betatab = dtable(ctx, beta.data(), nr);
   {
+    std::vector<double> lt((size_t)nr * FB_LIM_TAB, 0.0);
+    const double rs = p->indirecttermsmoothing;
+    for (int i = 0; i < nr; i++) {
+      double *t = &lt[(size_t)i * FB_LIM_TAB];
+      const double a = dxrad[i], b = dxth_cfl[i], m = (b < a) ? b : a, d2 = g.rmed[i] * g.rmed[i] + rs * rs;
+      t[0] = a;
+      t[1] = b;
+      t[2] = m;
+      t[3] = 1.0 / a;
+      t[4] = 1.0 / b;
+      t[5] = 1.0 / m;
+      t[6] = mindx2[i];
+      t[7] = 1.0 / mindx2[i];
+      t[8] = 1.0 / d2 / sqrt(d2);
+    }
+    k.lim_tab = dtable(ctx, lt.data(), lt.size());
+    if (!k.lim_tab) { fb_destroy(ctx); return FB_ERR_NOMEM; }
+  }
+  {
     std::vector<double> st((size_t)nr * FB_SRC_TAB);
     fb_source_table(&g, invdxth.data(), p15.data(), cs_ring.data(), st.data());
     k.src_tab = dtable(ctx, st.data(), st.size());
@@ -420,6 +439,8 @@ extern "C" int fb_create(const fb_params *p, const double *radii, fb_ctx **out)
   k.pmax = p->pmax;
   k.dphi = (p->pmax - p->pmin) / (double)ns;
   k.invdphi = 1.0 / k.dphi;
+  k.invspan = 1.0 / (p->pmax - p->pmin);
+  k.invns = 1.0 / (double)ns;
   k.omega_frame = p->omegaframe;
   k.corot = p->corotating;
   k.gamma = p->adiabaticindex;

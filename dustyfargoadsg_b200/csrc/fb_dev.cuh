@@ -16,7 +16,7 @@
 // (src/SourceEuler.c:333-460), advanced by a one-thread kernel so that the
 // whole substep stays on the device.
 struct fb_ctl {
-  double DT, dtemp, dt, dthydro, dtnbody;
+  double DT, dtemp, dt, invdt, dthydro, dtnbody;
   double physical_time, physical_time_initial, omega_frame;
   double mindt, maxdt, lost_mass;
   double disk_acc_x, disk_acc_y, disk_acc_alt_x, disk_acc_alt_y;
@@ -74,6 +74,7 @@ struct fb_lsa {
   double s[FB_LSA_MAX_MODES], cp[FB_LSA_MAX_MODES], sp[FB_LSA_MAX_MODES];
 };
 
+#define FB_LIM_TAB 10  // doubles per ring of KP::lim_tab
 #define FB_SRC_TAB 14  // doubles per ring of KP::src_tab
 
 // Everything a kernel needs, passed by value (well under the 32 KB limit).
@@ -126,11 +127,13 @@ struct KP {
   double *ringmin, *vmoy;
   double *vt_part;  // beta cooling: per ring, SubStep2's partial sums of vtheta (one per tile of k_sources)
   double *partials;
+  const double *lim_tab;  // FB_LIM_TAB per ring: see LimRing (fb_gas.cu)
   int n_partial_blocks;
   fb_ctl *ctl;
   int cap;  // most substeps of a DT
   // scalars
   double pmin, pmax, dphi, invdphi, omega_frame;
+  double invspan, invns;  // 1 / (pmax - pmin), 1 / nsec
   // frame corotating with the first planet (FRAME C): OmegaFrame changes
   // every substep and lives in the control block; kernels read it via omf()
   int corot;

@@ -23,10 +23,25 @@ int fb_pdl = 1;
 // per-cell kernels: CTAs of k.cell_bs azimuths (a ring segment) times rings
 static inline dim3 grid2d(const KP &k, int rings) { return dim3((k.ns + k.cell_bs - 1) / k.cell_bs, rings); }
 
+// The lengths of ring i that the time step's limits divide by, their
+// reciprocals (correctly rounded on the host, so that fb_quot's quotients are
+// the correctly rounded ones) and the star's smoothed 1/d^3.  As divisions in
+// every thread these constants cost more than the cells' own arithmetic.
+struct LimRing {
+  double dxrad, dxtheta, dxmin, rdxrad, rdxtheta, rdxmin, mindx2, rmindx2, invd3;
+};
+static __device__ __forceinline__ LimRing lim_ring(const KP &k, int i)
+{
+  const double2 *t = (const double2 *)(k.lim_tab + (size_t)i * FB_LIM_TAB);
+  const double2 a = t[0], b = t[1], c = t[2], d = t[3], e = t[4];
+  return {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x};
+}
+
 static __device__ __forceinline__ double min2(double a, double b) { return (b < a) ? b : a; }  // SourceEuler.c:293
 static __device__ __forceinline__ double max2(double a, double b) { return (b > a) ? b : a; }  // SourceEuler.c:300
 
 static __device__ __forceinline__ double dt_of(const KP &k, double dtov) { return dtov > 0.0 ? dtov : k.ctl->dt; }
+static __device__ __forceinline__ double invdt_of(const KP &k, double dtov) { return dtov > 0.0 ? 1.0 / dtov : k.ctl->invdt; }
 
 // ------------------------------------------------------------ reductions
 template <int BS>
@@ -183,13 +198,13 @@ __global__ void __launch_bounds__(CFL_BS, 4) k_cfl(KP k)
   const double *vt = k.vt + base, *vr = k.vr + base, *rho = k.rho + base;
   const bool cfl = (i >= 1);  // ConditionCFL's rings: One_or_active..Max_or_active-1
   if (i == 0 && tid == 0) planet_prelude(k, k.ctl);
-  const double rmi = k.rmed[i], surf = k.surf[i], rs = k.indirect_smoothing;
+  const double rmi = k.rmed[i], surf = k.surf[i];
+  const LimRing L = lim_ring(k, i);
 #if FB_FAST
   // fast build: every cell of the ring lies rmed[i] from the star, so the
   // smoothed 1/d^3 of the star's sums is the ring's (within a few ulp of
   // the reference's per-cell value): one root and two divisions per ring
-  const double dist2_ring = rmi * rmi + rs * rs;
-  const double invd3_ring = 1.0 / dist2_ring / sqrt(dist2_ring);
+  const double invd3_ring = L.invd3;
 #endif
   // ring sums: vtheta; ComputeForce (Force.c:77-253) for the star (x = y = 0,
   // mass 0) with rsmoothing = INDIRECTTERMSMOOTHING (SourceEuler.c:482);
@@ -199,11 +214,10 @@ __global__ void __launch_bounds__(CFL_BS, 4) k_cfl(KP k)
   // residual-velocity one are known before the ring mean; the sum under the
   // square root is evaluated in the reference's order once it is
   double *vtc = cfl_sm, *s12 = cfl_sm + ns, *s4 = cfl_sm + 2 * ns;
-  const double dxrad = k.dxrad[i], dxtheta = k.dxtheta_cfl[i];
+  const double dxrad = L.dxrad, dxtheta = L.dxtheta, rdxrad = L.rdxrad, rdxtheta = L.rdxtheta;
   // the quotients by the ring's constant lengths, each correctly rounded
   // through one reciprocal per ring
-  const double dxmin = min2(dxrad, dxtheta);
-  const double rdxmin = 1.0 / dxmin, rdxrad = 1.0 / dxrad, rdxtheta = 1.0 / dxtheta;
+  const double dxmin = L.dxmin, rdxmin = L.rdxmin;
   int negd = 0, nege = 0, bad = 0;
   for (int j = tid; j < ns; j += T) {
     const double vtj = vt[j], vrj = vr[j], dens = rho[j];
@@ -223,7 +237,7 @@ __global__ void __launch_bounds__(CFL_BS, 4) k_cfl(KP k)
     const double InvDist3 = invd3_ring;
 #else
     const double d2 = dx * dx + dy * dy;
-    const double dist2 = d2 + rs * rs;
+    const double dist2 = d2 + k.indirect_smoothing * k.indirect_smoothing;
     const double distance = sqrt(dist2);
     const double InvDist3 = 1.0 / dist2 / distance;
 #endif
@@ -264,11 +278,11 @@ __global__ void __launch_bounds__(CFL_BS, 4) k_cfl(KP k)
   }
   if (cfl) {
     const double viscosity = nu_ring(k, i);
-    const double invdt5 = (viscosity != 0.0) ? viscosity * 4.0 / k.mindx2[i] : 1e-10;
+    const double invdt5 = (viscosity != 0.0) ? fb_quot(viscosity * 4.0, L.mindx2, L.rmindx2) : 1e-10;
     // thermal diffusion's limit (SourceEuler.c:1411-1428): entropy
     // diffusion's per ring; explicit radiative diffusion's per cell (below),
     // which replaces it when both are on
-    const double invdt6_ring = (k.energy && k.ent_diff) ? k.diffusivity * 4.0 / k.mindx2[i] : 1e-10;
+    const double invdt6_ring = (k.energy && k.ent_diff) ? fb_quot(k.diffusivity * 4.0, L.mindx2, L.rmindx2) : 1e-10;
     // the ring's limit is the smallest CFLSECURITY / sqrt(S) over its cells;
     // a correctly rounded square root and quotient are monotone, so it is
     // the limit of the largest S, to the last bit: one root and one division
@@ -517,7 +531,9 @@ static __device__ void planet_prelude(const KP &k, fb_ctl *c)
       double RRoche = PlanetDistance * pow((1.0 / 3.0 * mplanet), 1.0 / 3.0);
       smoothing = RRoche * k.rochesmoothing;
     } else {
-      smoothing = k.thicksmoothing * dev_aspect_ratio(k, PlanetDistance) * pow(PlanetDistance, 1.0 + k.flaringindex);
+      // pow(x, 1.0) is x: no call where the disc does not flare (1.5 us on the time step's path)
+      smoothing = k.thicksmoothing * dev_aspect_ratio(k, PlanetDistance) *
+                  (k.flaringindex == 0.0 ? PlanetDistance : pow(PlanetDistance, 1.0 + k.flaringindex));
     }
     c->pot_m[p] = mplanet;
     c->pot_x[p] = xplanet;
@@ -591,6 +607,7 @@ static __device__ void controller_body(const KP &k, double *sh, fb_ctl *c)
   const double dt = min2(dthydro, dtnbody);
   c->dthydro = dthydro;
   c->dt = dt;
+  c->invdt = 1.0 / dt;
   c->dtemp += dt;
   if (dt < c->mindt) c->mindt = dt;
   if (dt > c->maxdt) c->maxdt = dt;
@@ -932,15 +949,29 @@ __global__ void __launch_bounds__(FB_BS2) k_substep3(KP k, int nparts)
 {
   fb_grid_dependency();
   const int ns = k.ns, nr = k.nr;
-  const int i = blockIdx.y, j = blockIdx.x * blockDim.x + threadIdx.x;
-  // the ring sum of vtheta from the tiles' partial sums, by each warp in the
-  // same order (a lane's strided sums, then across lanes)
-  double vsum = 0.0;
-  if (k.beta_cooling) {
-    for (int b = threadIdx.x & 31; b < nparts; b += 32) vsum += k.vt_part[(size_t)i * nparts + b];
-    for (int o = 16; o > 0; o >>= 1) vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
+  const int i = blockIdx.y;
+  int j = blockIdx.x * blockDim.x + threadIdx.x;
+  // beta cooling (SourceEuler.c:1196-1203): 1 + dt over the ring's cooling time
+  // and its reciprocal, by the CTA's first warp (five divisions that every
+  // thread would repeat): the ring sum of vtheta from the tiles' partial sums,
+  // a lane's strided sums, then across lanes
+  __shared__ double cool[2];
+  const double dt = k.ctl->dt;
+  if (k.beta_cooling && !k.thermal_cooling && threadIdx.x < 32) {
+    double omega = 0.0;
+    for (int b = threadIdx.x; b < nparts; b += 32) omega += k.vt_part[(size_t)i * nparts + b];
+    for (int o = 16; o > 0; o >>= 1) omega += __shfl_xor_sync(0xffffffffu, omega, o);
+    omega /= (double)ns;
+    omega /= k.rmed[i];
+    const double coolingtime = k.betatab[i] / omega;
+    const double d2 = 1.0 + dt / coolingtime;
+    if (threadIdx.x == 0) {
+      cool[0] = d2;
+      cool[1] = 1.0 / d2;
+    }
   }
-  if (j >= ns) return;
+  const bool cell = (j < ns);  // the others only meet the barrier below
+  if (!cell) j = ns - 1;
   const size_t l = (size_t)i * ns + j;
   const bool heat = k.viscous_heating;
   const Stress st = stress_at(k, k.vr_mid, k.vt_mid, i, j, heat);
@@ -953,16 +984,7 @@ __global__ void __launch_bounds__(FB_BS2) k_substep3(KP k, int nparts)
     r2 = k.rho[l + 2 * ns];
   }
   const double el = k.e_mid[l], rl = k.rho[l];
-  const double dt = k.ctl->dt;
-  const bool keep = k.ctl->done || k.ctl->status || k.ctl->substeps >= k.cap;
-  double coolfac = 0.0;
-  if (k.beta_cooling) {
-    double omega = vsum;
-    omega /= (double)ns;
-    omega /= k.rmed[i];
-    double coolingtime = k.betatab[i] / omega;
-    coolfac = coolingtime;
-  }
+  const bool keep = cell && (k.ctl->done || k.ctl->status || k.ctl->substeps >= k.cap);
   if (keep) k.divv[l] = st.div;
   double vh = 0.0;
   if (heat) {
@@ -1018,11 +1040,11 @@ __global__ void __launch_bounds__(FB_BS2) k_substep3(KP k, int nparts)
       en = num / den;
     }
     if (k.beta_cooling) {
-      const double d2 = 1.0 + dt / coolfac;  // one per ring: the quotient through its reciprocal
-      en = fb_quot(en, d2, 1.0 / d2);
+      __syncthreads();
+      en = fb_quot(en, cool[0], cool[1]);
     }
   }
-  k.e[l] = en;
+  if (cell) k.e[l] = en;
 }
 
 // ComputeOpacities (SourceEuler.c:1608-1701): Bell & Lin (1994) opacities of
@@ -1856,7 +1878,7 @@ static __device__ __forceinline__ void azr_load(const double *p, double (&v)[E])
 // The ring's entries of the 1-D tables, loaded together with the ring's
 // fields (not one by one where the arithmetic first needs them).
 struct AzrTab {
-  double invrmed, rmed, dxtheta, invdxtheta, rsup, rinf, surf, vthetamed, energymed;
+  double invrmed, rmed, dxtheta, invdxtheta, rsup, rinf, invsurf, vthetamed, energymed;
 };
 static __device__ __forceinline__ AzrTab azr_tab(const KP &k, int i)
 {
@@ -1867,10 +1889,21 @@ static __device__ __forceinline__ AzrTab azr_tab(const KP &k, int i)
   t.invdxtheta = k.invdxtheta[i];
   t.rsup = k.rsup[i];
   t.rinf = k.rinf[i];
-  t.surf = k.surf[i];
+  t.invsurf = k.invsurf[i];
   t.vthetamed = k.vthetamed ? k.vthetamed[i] : 0.0;
   t.energymed = (k.energy && k.energymed) ? k.energymed[i] : 0.0;
   return t;
+}
+
+// Ring cell of a tile's cell c, -AZT_LEFT <= c < ns + 32 E: one turn at most
+// unless the ring is shorter than a tile (an integer remainder per cell was 6%
+// of the pass's instructions).
+template <int E>
+static __device__ __forceinline__ int azt_wrap(int c, int ns)
+{
+  if (ns >= 32 * E) return (c < 0) ? c + ns : (c >= ns) ? c - ns : c;
+  c %= ns;
+  return (c < 0) ? c + ns : c;
 }
 
 // Neighbour values within one warp only (the tile variant): lane 0's left
@@ -1891,7 +1924,7 @@ static __device__ __forceinline__ void azt_exchange(const double *sL, double *rL
 // ring cell of the warp's first loaded cell plus lane E (any integer: taken
 // modulo nsec), the ring mean vmed_in given, no barrier at all.
 template <int NQ, int E, bool TILE, class Out>
-static __device__ __forceinline__ void azr_ring(const KP &k, double dt, int i, const AzrTab &tb,
+static __device__ __forceinline__ void azr_ring(const KP &k, double dt, double dtov, int i, const AzrTab &tb,
                                                 double (&q0)[NQ][E], const double (&vt)[E], const double (&vs)[E],
                                                 double vmed_in, int c0, double *sh,
                                                 double (*hal)[2][AZR_MAXW][AZR_NV], int &xb, Out out)
@@ -1908,7 +1941,10 @@ static __device__ __forceinline__ void azr_ring(const KP &k, double dt, int i, c
       azr_exchange<NL, NR>(hal, xb, lane, w, wl, wr, sL, rL, sR, rR);       \
   } while (0)
   // ComputeThetaElongations / ComputeAverageThetaVelocities / ComputeResiduals
-  const double invdt = 1.0 / dt;
+  // The launch's and the ring's constants come from the host or the controller
+  // (reciprocals correctly rounded, quotients by them exact through fb_quot):
+  // as divisions in every thread they were a tenth of the pass's instructions.
+  const double invdt = invdt_of(k, dtov);
   double VMed = vmed_in;
   if (!TILE) {
     double s = 0.0;
@@ -1918,11 +1954,11 @@ static __device__ __forceinline__ void azr_ring(const KP &k, double dt, int i, c
       s += elong * invdt;
     }
     s = block_sum_dyn(s, sh);
-    VMed = s / (double)ns;
+    VMed = fb_quot(s, (double)ns, k.invns);
   }
   // ComputeConstantResidual (TransportEuler.c:310-348)
-  const double dpinvns = (k.pmax - k.pmin) / (double)ns;
-  const double Ntilde = VMed * tb.invrmed * dt * (double)ns / (k.pmax - k.pmin);
+  const double dpinvns = k.dphi;  // (pmax - pmin) / ns
+  const double Ntilde = fb_quot(VMed * tb.invrmed * dt * (double)ns, k.pmax - k.pmin, k.invspan);
   const double Nround = floor(Ntilde + 0.5);
   const long nshift = (long)Nround;
   double vconst = (Ntilde - Nround) * tb.rmed * invdt * dpinvns;
@@ -1936,7 +1972,7 @@ static __device__ __forceinline__ void azr_ring(const KP &k, double dt, int i, c
   if (!k.fast_transport) vconst = 0.0;
   const double dxtheta = tb.dxtheta, invdxtheta = tb.invdxtheta;
   const double dxrad = (tb.rsup - tb.rinf) * dt;
-  const double invsurf = 1.0 / tb.surf;
+  const double invsurf = tb.invsurf;
   for (int pass = 0; pass < 2; pass++) {
     const bool uniform = (pass == 1);
     if (uniform && !k.fast_transport) break;  // NoSplitAdvection: no update
@@ -2063,15 +2099,13 @@ static __device__ __forceinline__ void azr_ring(const KP &k, double dt, int i, c
   for (int e = 0; e < E; e++) {
     int p;
     if (TILE) {
-      int g = (c0 + e) % ns;
-      if (g < 0) g += ns;
-      p = g + shift;
+      p = azt_wrap<E>(c0 + e, ns) + shift;
     } else {
       p = c0 + e + shift;
     }
     if (p >= ns) p -= ns;
     const double tpm = (e == 0) ? xl[0] : q0[2][e - 1], rm = (e == 0) ? xl[1] : q0[RH][e - 1];
-    double v = (tpm + q0[3][e]) / (q0[RH][e] + rm + 1e-20) / rmi - rmi * omf(k);
+    double v = fb_quot((tpm + q0[3][e]) / (q0[RH][e] + rm + 1e-20), rmi, tb.invrmed) - rmi * omf(k);
     if (subkep) v = tb.vthetamed - rmi * omf(k);
     double en = 0.0;
     if (NQ == 6) {
@@ -2105,7 +2139,7 @@ __global__ void __launch_bounds__(MT) k_transport_azimuthal_reg(KP k, double dto
 #pragma unroll
   for (int e = 0; e < E; e++) vs[e] = k.vt_src[base + tid + e * T];
   const AzrTab tb = azr_tab(k, i);
-  azr_ring<NQ, E, false>(k, dt, i, tb, q0, vt, vs, 0.0, c0, sh, hal, xb,
+  azr_ring<NQ, E, false>(k, dt, dtov, i, tb, q0, vt, vs, 0.0, c0, sh, hal, xb,
                          [&](int, int p, double v, double r, double a, double b, double en) {
                     k.vt[base + p] = v;
                     k.rho_t[base + p] = r;
@@ -2143,7 +2177,7 @@ __global__ void __launch_bounds__(1024) k_azi_vmed(KP k, double dtov)
   const double dt = dt_of(k, dtov);
   const int i = blockIdx.x, ns = k.ns, T = blockDim.x;
   const double *vt = k.vt_src + (size_t)i * ns;
-  const double invdt = 1.0 / dt;
+  const double invdt = invdt_of(k, dtov);
   double s = 0.0;
   for (int j = threadIdx.x; j < ns; j += T) {
     double elong = vt[j] * dt;
@@ -2170,8 +2204,7 @@ __global__ void __launch_bounds__(AZT_WPC * 32, MINB) k_transport_azimuthal_tile
   double q0[NQ][E], vt[E], vs[E];
 #pragma unroll
   for (int e = 0; e < E; e++) {
-    int g = (c0 + e) % ns;
-    if (g < 0) g += ns;
+    const int g = azt_wrap<E>(c0 + e, ns);
     const size_t l = base + g;
 #pragma unroll
     for (int q = 0; q < NQ; q++) q0[q][e] = (q < 2 ? k.azt_buf[q] : k.q[q])[l];
@@ -2182,7 +2215,7 @@ __global__ void __launch_bounds__(AZT_WPC * 32, MINB) k_transport_azimuthal_tile
   const double vmed = k.azt_vmed[i];
   int xb = 0;
   const int m0 = lane * E - AZT_LEFT, tcell = t * CO;  // tile cell of own cell e: m0 + e
-  azr_ring<NQ, E, true>(k, dt, i, tb, q0, vt, vs, vmed, c0, nullptr, nullptr, xb,
+  azr_ring<NQ, E, true>(k, dt, dtov, i, tb, q0, vt, vs, vmed, c0, nullptr, nullptr, xb,
                         [&](int e, int p, double v, double r, double a, double b, double en) {
                           const int m = m0 + e;
                           if (m < 0 || m >= CO || tcell + m >= ns) return;
@@ -2298,7 +2331,7 @@ __global__ void __launch_bounds__(MT) k_transport_azimuthal_staged(KP k, double 
     }
     __syncthreads();  // every row read: the buffer takes the results
     double *o = buf + (size_t)b * NB * ns;
-    azr_ring<NQ, E, false>(k, dt, i, tb, q0, vt, vs, 0.0, tid * E, sh, hal, xb,
+    azr_ring<NQ, E, false>(k, dt, dtov, i, tb, q0, vt, vs, 0.0, tid * E, sh, hal, xb,
                            [&](int, int p, double v, double r, double a, double bb, double en) {
                       o[p] = v;
                       o[(size_t)ns + p] = r;
@@ -3100,13 +3133,13 @@ __global__ void __launch_bounds__(FB_BS) k_damping(KP k, double dtov)
       const int j = j0 + u * FB_BS;
       if (j >= ns) continue;
       const size_t l = base + j;
+      const double vtn = zero_here ? vtheta0 : fb_quot(vt[u] + lambda * vtheta0, den, rden);
+      k.vt[l] = vtn;
       if (zero_here) {
         k.vr[l] = 0.0;
         k.rho[l] = dens0;
-        k.vt[l] = vtheta0;
       } else {
         k.vr[l] = fb_quot(vr[u] + lambda * vrad0, den, rden);
-        k.vt[l] = fb_quot(vt[u] + lambda * vtheta0, den, rden);
         k.rho[l] = fb_quot(rh[u] + lambda * dens0, den, rden);
       }
       if (k.energy) k.e[l] = fb_quot(en[u] + lambda * energ0, den, rden);
@@ -3208,11 +3241,11 @@ __global__ void __launch_bounds__(MT, 2) k_finish(KP k, int fuse_cs, cudaGraphCo
         m[4] += vp[e];
       }
       block_sums<5>(m, sh);
-      vrad0 = m[0] / (double)ns;
-      vtheta0 = m[1] / (double)ns;
-      dens0 = m[2] / (double)ns;
-      energ0 = m[3] / (double)ns;
-      vradp0 = m[4] / (double)ns;
+      vrad0 = fb_quot(m[0], (double)ns, k.invns);
+      vtheta0 = fb_quot(m[1], (double)ns, k.invns);
+      dens0 = fb_quot(m[2], (double)ns, k.invns);
+      energ0 = fb_quot(m[3], (double)ns, k.invns);
+      vradp0 = fb_quot(m[4], (double)ns, k.invns);
     } else {
       vtheta0 = k.vthetamed[i] - k.rmed[i] * omf(k);
       vrad0 = k.vradmed[i];
@@ -3254,15 +3287,14 @@ __global__ void __launch_bounds__(MT, 2) k_finish(KP k, int fuse_cs, cudaGraphCo
   }
   __syncthreads();
   // ---- ConditionCFL, ring sums and DetectCrash: see k_cfl
-  const double rmi = k.rmed[i], surf = k.surf[i], rs = k.indirect_smoothing;
+  const double rmi = k.rmed[i], surf = k.surf[i];
+  const LimRing L = lim_ring(k, i);
 #if FB_FAST
-  const double dist2_ring = rmi * rmi + rs * rs;
-  const double invd3_ring = 1.0 / dist2_ring / sqrt(dist2_ring);
+  const double invd3_ring = L.invd3;
 #endif
   double s[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  const double dxrad = k.dxrad[i], dxtheta = k.dxtheta_cfl[i];
-  const double dxmin = min2(dxrad, dxtheta);
-  const double rdxmin = 1.0 / dxmin, rdxrad = 1.0 / dxrad, rdxtheta = 1.0 / dxtheta;
+  const double dxrad = L.dxrad, dxtheta = L.dxtheta, rdxrad = L.rdxrad, rdxtheta = L.rdxtheta;
+  const double dxmin = L.dxmin, rdxmin = L.rdxmin;
   int negd = 0, nege = 0, bad = 0;
 #pragma unroll
   for (int e = 0; e < E; e++) {
@@ -3281,7 +3313,7 @@ __global__ void __launch_bounds__(MT, 2) k_finish(KP k, int fuse_cs, cudaGraphCo
 #if FB_FAST
     const double InvDist3 = invd3_ring;
 #else
-    const double dist2 = xc * xc + yc * yc + rs * rs;
+    const double dist2 = xc * xc + yc * yc + k.indirect_smoothing * k.indirect_smoothing;
     const double distance = sqrt(dist2);
     const double InvDist3 = 1.0 / dist2 / distance;
 #endif
@@ -3309,7 +3341,7 @@ __global__ void __launch_bounds__(MT, 2) k_finish(KP k, int fuse_cs, cudaGraphCo
     vp[e] = invdt4 * invdt4;
   }
   block_sums<7>(s, sh);
-  const double vmoy = s[0] / (double)ns;
+  const double vmoy = fb_quot(s[0], (double)ns, k.invns);
   if (tid == 0) {
     k.vmoy[i] = vmoy;
     double *pp = k.partials + (size_t)i * 5;  // summed by the controller in ring order
@@ -3323,8 +3355,8 @@ __global__ void __launch_bounds__(MT, 2) k_finish(KP k, int fuse_cs, cudaGraphCo
   }
   if (i >= 1) {
     const double viscosity = nu_ring(k, i);
-    const double invdt5 = (viscosity != 0.0) ? viscosity * 4.0 / k.mindx2[i] : 1e-10;
-    const double invdt6 = (ENERGY && k.ent_diff) ? k.diffusivity * 4.0 / k.mindx2[i] : 1e-10;
+    const double invdt5 = (viscosity != 0.0) ? fb_quot(viscosity * 4.0, L.mindx2, L.rmindx2) : 1e-10;
+    const double invdt6 = (ENERGY && k.ent_diff) ? fb_quot(k.diffusivity * 4.0, L.mindx2, L.rmindx2) : 1e-10;
     double smax = -1.0;
 #pragma unroll
     for (int e = 0; e < E; e++) {

@@ -178,6 +178,9 @@ extern "C" int fb_transport_noalloc(const fb_params *p, double *dens, double *vr
   k.ctl = d.ctl;
   k.pmin = p->pmin;
   k.pmax = p->pmax;
+  k.dphi = (p->pmax - p->pmin) / (double)ns;
+  k.invspan = 1.0 / (p->pmax - p->pmin);
+  k.invns = 1.0 / (double)ns;
   k.omega_frame = p->omegaframe;
   k.energy = p->energy_equation;
   k.fast_transport = p->fast_transport;
