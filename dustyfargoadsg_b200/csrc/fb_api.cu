@@ -394,13 +394,18 @@ extern "C" int fb_create(const fb_params *p, const double *radii, fb_ctx **out)
   k.damp_lam = dtable(ctx, dlam.data(), nr);
   k.damp_tau = dtable(ctx, dtau.data(), nr);
   {
+    // the damping rings, then the others and ring nr
+    const int nd = (int)drings.size();
+    std::vector<int> list = drings;
+    for (int i = 0, q = 0; i <= nr; i++)
+      if (q < nd && drings[q] == i) q++;
+      else list.push_back(i);
     int *d = NULL;
-    if (!drings.empty()) {
-      cudaMalloc(&d, drings.size() * sizeof(int));
-      cudaMemcpy(d, drings.data(), drings.size() * sizeof(int), cudaMemcpyHostToDevice);
-      ctx->allocs.push_back(d);
-    }
+    if (cudaMalloc(&d, list.size() * sizeof(int)) != cudaSuccess) { fb_destroy(ctx); return FB_ERR_NOMEM; }
+    cudaMemcpy(d, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice);
+    ctx->allocs.push_back(d);
     k.damp_rings = d;
+    k.calm_rings = d + nd;
     k.n_damp_rings = (int)drings.size();
   }
   k.vh_l1 = log(g.rmed[0] / g.rmed[1]);
@@ -869,7 +874,12 @@ static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NU
     if (fb_azi_launches(kt) == 2) STAGE(ST_TVMED, 1, fb_launch_azi_vmed(kt, 0.0, s));
     STAGE(ST_TAZI, 1, fb_launch_transport_azimuthal(kt, 0.0, s, true));
   }
-  if (!at_end) STAGE(ST_TVR, 1, fb_launch_transport_vr(k, s));
+  // walls: vr and the damping in one launch, where any ring damps
+  const bool vr_damp = !at_end && !edges_other_than_wall(k) && k.evanescent && k.n_damp_rings > 0;
+  if (vr_damp)
+    STAGE(ST_TVR, 1, fb_launch_vr_damping(k, s));
+  else if (!at_end)
+    STAGE(ST_TVR, 1, fb_launch_transport_vr(k, s));
   if (edges_other_than_wall(k)) {
     // ApplyBoundaryCondition's other edges (SideEuler.c:1102-1131); the
     // non-reflecting edge reads the planets' new positions and, with the
@@ -878,7 +888,7 @@ static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NU
     if (k.non_reflecting && k.energy) STAGE(ST_TVR, 1, fb_launch_soundspeed(k, 0, s));
     STAGE(ST_TVR, 1, fb_launch_edges(k, s));
   }
-  if (!at_end && k.evanescent && k.n_damp_rings > 0) STAGE(ST_DAMP, 1, fb_launch_damping(k, 0.0, s));
+  if (!at_end && !vr_damp && k.evanescent && k.n_damp_rings > 0) STAGE(ST_DAMP, 1, fb_launch_damping(k, 0.0, s));
   if (!ctx->has_dust) cudaStreamWaitEvent(s, ctx->ev_planets, 0);
   if (dust_branch) cudaStreamWaitEvent(s, ctx->ev_dust_end, 0);
   if (at_end) {

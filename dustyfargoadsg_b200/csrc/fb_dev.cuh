@@ -121,6 +121,7 @@ struct KP {
   const double *damp_lam;  // damping*damping per ring (0 outside the zones)
   const double *damp_tau;  // DAMPINGTODYNAMICALTIMERATIO*pow(Rmed,1.5)
   const int *damp_rings;   // list of rings inside the wave-killing zones
+  const int *calm_rings;   // the others, then ring nr
   int n_damp_rings;
   double vh_l1, vh_l2;     // log(r/rip), log(rip/ri2p) for ViscHeat at i=0
   // CFL / reductions
@@ -398,6 +399,7 @@ void fb_launch_opacity(const KP &k, int constant, double imposed, double factor,
                        double unit_mass, double inv_l3, double conv, cudaStream_t s);
 void fb_launch_floors_boundary(const KP &k, cudaStream_t s);
 void fb_launch_damping(const KP &k, double dt_override, cudaStream_t s);
+void fb_launch_vr_damping(const KP &k, cudaStream_t s);  // both in one launch (discs with walls)
 // the end of a substep in one pass (discs with walls, small grids): vr, floors,
 // walls, damping, the next substep's CFL limits and controller, with fuse_cs
 // its sound speed, and the loop condition h (if any)

@@ -3152,6 +3152,127 @@ void fb_launch_damping(const KP &k, double dt_override, cudaStream_t s)
   if (k.n_damp_rings > 0) fb_launch(k_damping, k.n_damp_rings, FB_BS, 0, s, k, dt_override);
 }
 
+// ------------------------------------------- vr, floors, walls and damping
+// k_transport_vr and k_damping in one launch (discs with walls): the first CTAs
+// take a damping ring each, from the transport's outputs through vr, floors
+// and walls to the damped state (the ring's vr and density wait in shared
+// memory for the ring means), the others the cells of the other rings as
+// k_transport_vr does.  Few rings damp and each is a chain of reductions, so
+// as a launch of its own k_damping left most of the GPU idle; here the other
+// rings' cells fill it.
+#define VD_BS 256
+__global__ void __launch_bounds__(VD_BS) k_vr_damping(KP k, int segs)
+{
+  fb_grid_dependency();
+  __shared__ double shm[4 * 32];
+  extern __shared__ double vd_sm[];
+  const int ns = k.ns, nr = k.nr, tid = threadIdx.x;
+  const int wall = k.wall, floors = k.add_floors;
+  // ComputeVelocities (TransportEuler.c:531-536) at interface ring ii, azimuth j
+  auto vr_at = [&](int ii, int j) -> double {
+    if (ii == 0) return 0.0;
+    const size_t m = (size_t)ii * ns + j;
+    return (k.q[0][m - ns] + k.q[1][m]) / (k.rho_t[m] + k.rho_t[m - ns] + 1e-20);
+  };
+  // vr and density of ring i after floors (SourceEuler.c:2506) and walls
+  // (SideEuler.c:1047-1099)
+  auto cell = [&](int i, int j, double &v, double &d) {
+    d = k.rho_t[(size_t)i * ns + j];
+    const int src = !wall ? i : i == 0 ? 2 : (i == 1 || i == nr - 1) ? 0 : i;
+    v = vr_at(src, j);
+    if (wall && i == 0) v = -v;
+    if (floors && d < k.floordens) d = k.floordens;
+    if (wall && (i <= 1 || i >= nr - 2)) d = k.sigmamed[i];
+  };
+  if ((int)blockIdx.x >= k.n_damp_rings) {
+    const int b = blockIdx.x - k.n_damp_rings, q = b / segs, j = (b - q * segs) * VD_BS + tid;
+    if (b == 0 && tid < 32) lost_mass_sum(k);
+    if (j >= ns) return;
+    const int i = k.calm_rings[q];  // the rings that do not damp, then ring nr
+    const size_t l = (size_t)i * ns + j;
+    if (i == nr) {  // zero without the wall since SubStep2 (k_sources)
+      if (wall) k.vr[l] = -vr_at(nr - 2, j);
+      return;
+    }
+    double v, d;
+    cell(i, j, v, d);
+    k.rho[l] = d;
+    k.vr[l] = v;
+    return;
+  }
+  // EvanescentBoundary (SideEuler.c:796-950): see k_damping
+  const int i = k.damp_rings[blockIdx.x];
+  const size_t base = (size_t)i * ns;
+  double *vs = vd_sm, *ds = vd_sm + ns;
+  const double lambda = k.damp_lam[i] * k.ctl->dt / k.damp_tau[i];
+  double m[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int j0 = tid; j0 < ns; j0 += 2 * VD_BS) {  // two cells' chains side by side
+    double v[2], d[2], vt[2] = {0.0, 0.0}, en[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const int j = j0 + u * VD_BS;
+      if (j >= ns) continue;
+      cell(i, j, v[u], d[u]);
+      vt[u] = k.vt[base + j];
+      en[u] = k.e[base + j];
+    }
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const int j = j0 + u * VD_BS;
+      if (j >= ns) continue;
+      vs[j] = v[u];
+      ds[j] = d[u];
+      m[0] += v[u];
+      m[1] += vt[u];
+      m[2] += d[u];
+      m[3] += en[u];
+    }
+  }
+  double vrad0, vtheta0, dens0, energ0;
+  if (k.damp_axi) {
+    block_sums<4>(m, shm);
+    vrad0 = fb_quot(m[0], (double)ns, k.invns);
+    vtheta0 = fb_quot(m[1], (double)ns, k.invns);
+    dens0 = fb_quot(m[2], (double)ns, k.invns);
+    energ0 = fb_quot(m[3], (double)ns, k.invns);
+  } else {
+    vtheta0 = k.vthetamed[i] - k.rmed[i] * omf(k);
+    vrad0 = k.vradmed[i];
+    dens0 = k.sigmamed[i];
+    energ0 = k.energymed[i];
+  }
+  const int zero_here = k.zero_vrad &&
+      (((k.rmed[i] < k.wkzrmin) && (i == 0 || i == 1)) || ((k.rmed[i] > k.wkzrmax) && (i == nr - 1)));
+  const double den = 1.0 + lambda, rden = 1.0 / den;
+  for (int j0 = tid; j0 < ns; j0 += RING_U * VD_BS) {
+    double vt[RING_U], en[RING_U];
+#pragma unroll
+    for (int u = 0; u < RING_U; u++) {
+      const int j = j0 + u * VD_BS;
+      if (j < ns) {
+        vt[u] = k.vt[base + j];
+        en[u] = k.energy ? k.e[base + j] : 0.0;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < RING_U; u++) {
+      const int j = j0 + u * VD_BS;
+      if (j >= ns) continue;
+      const size_t l = base + j;
+      k.vr[l] = zero_here ? 0.0 : fb_quot(vs[j] + lambda * vrad0, den, rden);
+      k.rho[l] = zero_here ? dens0 : fb_quot(ds[j] + lambda * dens0, den, rden);
+      k.vt[l] = zero_here ? vtheta0 : fb_quot(vt[u] + lambda * vtheta0, den, rden);
+      if (k.energy) k.e[l] = fb_quot(en[u] + lambda * energ0, den, rden);
+    }
+  }
+}
+
+void fb_launch_vr_damping(const KP &k, cudaStream_t s)
+{
+  const int segs = (k.ns + VD_BS - 1) / VD_BS, calm = k.nr + 1 - k.n_damp_rings;
+  fb_launch(k_vr_damping, k.n_damp_rings + calm * segs, VD_BS, 2 * (size_t)k.ns * sizeof(double), s, k, segs);
+}
+
 // ------------------------------------------------------------ end of a substep
 // ComputeVelocities' radial part, floors and walls (k_transport_vr), the
 // Stockholm damping (k_damping), the next substep's ConditionCFL with the
@@ -3534,6 +3655,7 @@ int fb_gas_prepare(int ns, int energy)
 #undef AZP_FNS
   {
     int rc = fb_allow_max_dynamic_smem((const void *)k_cfl);  // 3 nsec doubles of cell values
+    if (!rc) rc = fb_allow_max_dynamic_smem((const void *)k_vr_damping);  // 2 nsec
     if (rc) return rc;
   }
 #define AZS_FNS(NQ, EE)                                                                  \

@@ -17,7 +17,8 @@ pytestmark = pytest.mark.gpu
 
 TOL_DT = 1e-11
 SIZES = [(4, 16), (8, 26), (11, 27), (12, 28), (27, 53), (28, 54), (22, 81), (54, 55), (40, 200)]
-BIG = [(110, 540), (109, 541), (20, 384), (20, 385), (20, 1024), (20, 1025)]  # (110, 540): two rings per warp
+BIG = [(110, 540), (109, 541), (20, 384), (20, 385), (20, 1024), (20, 1025), (300, 40)]
+# (110, 540): two rings per warp of k_sources; (20, 1025), (300, 40): beyond k_finish
 
 
 def _cases():
