@@ -795,7 +795,8 @@ static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NU
     // applies its change before the gas update (SourceEuler.c:476-525)
     if (k.lsa) STAGE(ST_POT, 2, fb_launch_lsa_modes(k, s));
     STAGE(ST_CFL, 1, fb_launch_planets(k, NULL, s));
-    STAGE(ST_CFL, 1, fb_launch_correct_vtheta(k, s));
+    // (k_sources applies the change of the frame where it runs from the state)
+    if (k.self_gravity) STAGE(ST_CFL, 1, fb_launch_correct_vtheta(k, s));
     cudaEventRecord(ctx->ev_planets, s);
   } else {
     // the planets' step on a branch of its own: no gas kernel of the substep
@@ -884,8 +885,8 @@ static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NU
     // ApplyBoundaryCondition's other edges (SideEuler.c:1102-1131); the
     // non-reflecting edge reads the planets' new positions and, with the
     // energy equation, the sound speed of the transported state
+    // (k_transport_vr leaves it)
     if (k.non_reflecting && !ctx->has_dust) cudaStreamWaitEvent(s, ctx->ev_planets, 0);
-    if (k.non_reflecting && k.energy) STAGE(ST_TVR, 1, fb_launch_soundspeed(k, 0, s));
     STAGE(ST_TVR, 1, fb_launch_edges(k, s));
   }
   if (!at_end && !vr_damp && k.evanescent && k.n_damp_rings > 0) STAGE(ST_DAMP, 1, fb_launch_damping(k, 0.0, s));

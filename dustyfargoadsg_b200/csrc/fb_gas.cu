@@ -308,6 +308,52 @@ void fb_launch_cfl(const KP &k, cudaStream_t s)
   fb_launch(k_cfl, k.nr, cfl_threads(k.ns), 3 * (size_t)k.ns * sizeof(double), s, k);
 }
 
+// rk5 for one planet, its state in registers: the same operations in the same
+// order (terms that multiply zeroed stages left out).  The general form keeps
+// its arrays in shared memory and runs some 2,800 dependent instructions for a
+// single planet, about 20 us on the critical path of a corotating frame.
+static __device__ __forceinline__ void rk5_one_deriv(double x, double y, double vx, double vy, double mass, double dt,
+                                                     int indirect, double (&d)[4])
+{
+  const double r = sqrt(x * x + y * y);
+  const double s = -FB_G * 1.0 / r / r / r;
+  double ax = s * x, ay = s * y;
+  if (indirect) {
+    const double t = FB_G * mass / r / r / r;
+    ax -= t * x;
+    ay -= t * y;
+  }
+  d[0] = vx * dt;
+  d[1] = vy * dt;
+  d[2] = ax * dt;
+  d[3] = ay * dt;
+}
+static __device__ void rk5_one(double (&q)[4], double dt, double mass, int indirect)
+{
+  double k1[4], k2[4], k3[4], k4[4], k5[4], k6[4], p[4];
+  rk5_one_deriv(q[0], q[1], q[2], q[3], mass, dt, indirect, k1);
+#pragma unroll
+  for (int i = 0; i < 4; i++) p[i] = q[i] + 0.2 * k1[i];
+  rk5_one_deriv(p[0], p[1], p[2], p[3], mass, dt, indirect, k2);
+#pragma unroll
+  for (int i = 0; i < 4; i++) p[i] = q[i] + 0.075 * k1[i] + 0.225 * k2[i];
+  rk5_one_deriv(p[0], p[1], p[2], p[3], mass, dt, indirect, k3);
+#pragma unroll
+  for (int i = 0; i < 4; i++) p[i] = q[i] + 0.3 * k1[i] + -0.9 * k2[i] + 1.2 * k3[i];
+  rk5_one_deriv(p[0], p[1], p[2], p[3], mass, dt, indirect, k4);
+#pragma unroll
+  for (int i = 0; i < 4; i++) p[i] = q[i] + -11.0 / 54.0 * k1[i] + 2.5 * k2[i] + -70.0 / 27.0 * k3[i] + 35.0 / 27.0 * k4[i];
+  rk5_one_deriv(p[0], p[1], p[2], p[3], mass, dt, indirect, k5);
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    p[i] = q[i] + 1631.0 / 55296.0 * k1[i] + 175.0 / 512.0 * k2[i] + 575.0 / 13824.0 * k3[i] +
+           44275.0 / 110592.0 * k4[i] + 253.0 / 4096.0 * k5[i];
+  rk5_one_deriv(p[0], p[1], p[2], p[3], mass, dt, indirect, k6);
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    q[i] = q[i] + 37.0 / 378.0 * k1[i] + 250.0 / 621.0 * k3[i] + 125.0 / 594.0 * k4[i] + 512.0 / 1771.0 * k6[i];
+}
+
 // The planets' step of the substep, after the controller has set dt:
 // AdvanceSystemRK5 (Pframeforce.c:163-266) and RotatePsys (Psys.c:352-372).
 // One thread.  No other kernel of the substep reads the positions before the
@@ -326,7 +372,14 @@ __global__ void k_planets(KP k, fb_dust_ctl *dc, double thick, double aspect, do
   // 323-326): the first planet's position at the start of the substep
   const double xmark = (np > 0) ? c->px[0] : 0.0, ymark = (np > 0) ? c->py[0] : 0.0;
   // AdvanceSystemRK5 (Pframeforce.c:163-266)
-  if (!k.forced_circular) {
+  if (!k.forced_circular && np == 1) {
+    double q[4] = {c->px[0], c->py[0], c->pvx[0], c->pvy[0]};
+    rk5_one(q, dt, c->pm[0], k.indirect_term);
+    c->px[0] = q[0];
+    c->py[0] = q[1];
+    c->pvx[0] = q[2];
+    c->pvy[0] = q[3];
+  } else if (!k.forced_circular) {
     __shared__ RkWork rw;
     double *q0 = rw.q0, *q1 = rw.q1, *masses = rw.masses;
     for (int i = 0; i < np; i++) {
@@ -458,10 +511,10 @@ static __device__ void rk5(const double *q0, double dt, const double *masses, do
   // seeds them with the previous call's k6 (RungeKunta.c:73-75), which is
   // finite, so zeros give the same sums.
   double *k1 = w.k[0], *k2 = w.k[1], *k3 = w.k[2], *k4 = w.k[3], *k5 = w.k[4], *k6 = w.k[5];
-  for (int s = 0; s < 6; s++)
-    for (int i = 0; i < 4 * FB_MAX_PLANETS; i++) w.k[s][i] = 0.0;
   double *Dist = w.dist;
   const int m = 4 * n;
+  for (int s = 0; s < 6; s++)
+    for (int i = 0; i < m; i++) w.k[s][i] = 0.0;
   rk5_deriv(q0, masses, k1, n, dt, feelothers, indirect, Dist);
   for (int i = 0; i < m; i++) q1[i] = q0[i] + 0.2 * k1[i] + 0.0 * k2[i] + 0.0 * k3[i] + 0.0 * k4[i] + 0.0 * k5[i];
   rk5_deriv(q1, masses, k2, n, dt, feelothers, indirect, Dist);
@@ -2544,6 +2597,9 @@ __global__ void __launch_bounds__(FB_BS2) k_transport_vr(KP k)
     }
     k.rho[l] = d;
     k.vr[l] = v;
+    // the non-reflecting edges (and the next limits) read the sound speed of
+    // the transported state (ComputeSoundSpeed, SourceEuler.c:2323-2343)
+    if (k.non_reflecting && k.energy && !k.transport_only) k.cs[l] = sqrt(k.gamma * (k.gamma - 1.0) * k.e[l] / d);
   }
 }
 
@@ -2777,7 +2833,7 @@ void fb_launch_transport_vr(const KP &k, cudaStream_t s)
 __global__ void __launch_bounds__(EDGE_BS) k_edges(KP k)
 {
   fb_grid_dependency();
-  __shared__ double sh[32];
+  __shared__ double sh[3 * 32];
   const int ns = k.ns, nr = k.nr, tid = threadIdx.x, T = blockDim.x;
   const bool inner = (blockIdx.x == 0);
   double *rho = k.rho, *vr = k.vr, *vt = k.vt, *en = k.e;
@@ -2855,18 +2911,17 @@ __global__ void __launch_bounds__(EDGE_BS) k_edges(KP k)
     // :662-674 adiabatic)
     double cs1 = 0.0, d1 = 0.0, dangle;
     if (!k.energy) {
-      double cs0 = 0.0, d0 = 0.0;
+      double cs0 = 0.0;
       for (int j = tid; j < ns; j += T) {
         cs0 += cs[j];
         cs1 += cs[ns + j];
-        d0 += rho[j];
         d1 += rho[ns + j];
       }
-      cs0 = block_sum_dyn(cs0, sh) / (double)ns;
-      cs1 = block_sum_dyn(cs1, sh) / (double)ns;
-      d0 = block_sum_dyn(d0, sh) / (double)ns;  // dens0: unused without an accreting edge
-      d1 = block_sum_dyn(d1, sh) / (double)ns;
-      (void)d0;
+      double m[3] = {cs0, cs1, d1};  // dens0 is not used without an accreting edge
+      block_sums<3>(m, sh);
+      cs0 = m[0] / (double)ns;
+      cs1 = m[1] / (double)ns;
+      d1 = m[2] / (double)ns;
       dangle = (k.nrb_om1 - omega_in) / (.5 * (cs0 + cs1));
     } else {
       dangle = (k.nrb_om1 - omega_in) / (.5 * (k.nrb_csinit0 + k.nrb_csinit1));
@@ -2910,19 +2965,23 @@ __global__ void __launch_bounds__(EDGE_BS) k_edges(KP k)
       mean = block_sum_dyn(mean, sh) / (double)ns;
       for (int j = tid; j < ns; j += T) rho[j] += (k.sigmamed[0] - mean);
     } else {
+      // the density from the copied energy, then both shifted to their
+      // initial means: one reduction, the values at hand
       const double csinit0 = k.nrb_csinit0;
-      for (int j = tid; j < ns; j += T)
-        rho[j] = k.sigmamed[0] + (k.gamma - 1.0) * (en[j] - k.energymed[0]) / csinit0 / csinit0;
-      __syncthreads();
-      double mean = 0.0;
-      for (int j = tid; j < ns; j += T) mean += rho[j];
-      mean = block_sum_dyn(mean, sh) / (double)ns;
-      for (int j = tid; j < ns; j += T) rho[j] += (k.sigmamed[0] - mean);
-      __syncthreads();
-      mean = 0.0;
-      for (int j = tid; j < ns; j += T) mean += en[j];
-      mean = block_sum_dyn(mean, sh) / (double)ns;
-      for (int j = tid; j < ns; j += T) en[j] += (k.energymed[0] - mean);
+      auto dens_of = [&](double e) { return k.sigmamed[0] + (k.gamma - 1.0) * (e - k.energymed[0]) / csinit0 / csinit0; };
+      double m[2] = {0.0, 0.0};
+      for (int j = tid; j < ns; j += T) {
+        const double e = en[j];
+        m[0] += dens_of(e);
+        m[1] += e;
+      }
+      block_sums<2>(m, sh);
+      const double md = m[0] / (double)ns, me = m[1] / (double)ns;
+      for (int j = tid; j < ns; j += T) {
+        const double e = en[j];
+        rho[j] = dens_of(e) + (k.sigmamed[0] - md);
+        en[j] = e + (k.energymed[0] - me);
+      }
     }
   } else {
     // outermost planet inside the grid (SideEuler.c:718-728)
@@ -2936,18 +2995,14 @@ __global__ void __launch_bounds__(EDGE_BS) k_edges(KP k)
     }
     const int i = nr - 1;
     const size_t b1 = (size_t)(nr - 1) * ns, b2 = (size_t)(nr - 2) * ns;
-    double c2 = 0.0, c1 = 0.0, d1 = 0.0, d2 = 0.0;
+    double m[3] = {0.0, 0.0, 0.0};  // the density's mean on ring nr-1 is not used without an accreting edge
     for (int j = tid; j < ns; j += T) {
-      c2 += cs[b2 + j];
-      c1 += cs[b1 + j];
-      d1 += rho[b1 + j];
-      d2 += rho[b2 + j];
+      m[0] += cs[b2 + j];
+      m[1] += cs[b1 + j];
+      m[2] += rho[b2 + j];
     }
-    const double csnrm2 = block_sum_dyn(c2, sh) / (double)ns;
-    const double csnrm1 = block_sum_dyn(c1, sh) / (double)ns;
-    const double densnrm1 = block_sum_dyn(d1, sh) / (double)ns;  // unused without an accreting edge
-    const double densnrm2 = block_sum_dyn(d2, sh) / (double)ns;
-    (void)densnrm1;
+    block_sums<3>(m, sh);
+    const double csnrm2 = m[0] / (double)ns, csnrm1 = m[1] / (double)ns, densnrm2 = m[2] / (double)ns;
     double dangle = (k.nrb_omn2 - omega_out) / (.5 * (csnrm1 + csnrm2));
     dangle *= (k.rmed[nr - 1] - k.rmed[nr - 2]);
     const int i_angle = (int)(dangle / (k.pmax - k.pmin) * (double)ns + .5);
@@ -2958,6 +3013,7 @@ __global__ void __launch_bounds__(EDGE_BS) k_edges(KP k)
     // resolved and read before any cell is written.  A source outside rings
     // 3 .. nr-1 is not reproduced (FB_ERR_UNSUPPORTED).
     double *bufr = k.edge_buf + ns, *bufe = k.edge_buf + 2 * (size_t)ns;
+    double sums[2] = {0.0, 0.0};
     int bad = 0;
     for (int j = tid; j < ns; j += T) {
       const size_t l = (size_t)j + b1;
@@ -2984,8 +3040,11 @@ __global__ void __launch_bounds__(EDGE_BS) k_edges(KP k)
         bad = 1;
         src = (long)l;
       }
-      bufr[j] = rho[src];
-      bufe[j] = en[src];
+      const double rs = rho[src], es = en[src];
+      bufr[j] = rs;
+      bufe[j] = es;
+      sums[0] += rs;
+      sums[1] += es;
       const double vr_med = (!k.energy) ? csnrm1 * (rho[l - ns] - densnrm2) / densnrm2
                                         : cs[l] * (rho[l - ns] - densnrm2) / densnrm2;
       vr[l] = 2. * vr_med - vr[l - ns];
@@ -2994,20 +3053,13 @@ __global__ void __launch_bounds__(EDGE_BS) k_edges(KP k)
       if (tid == 0) k.ctl->status = FB_ERR_UNSUPPORTED;
       return;
     }
+    // ring nr-1 takes the copies, shifted to its initial means
+    block_sums<2>(sums, sh);
+    const double md = sums[0] / (double)ns, me = sums[1] / (double)ns;
     for (int j = tid; j < ns; j += T) {
-      rho[b1 + j] = bufr[j];
-      en[b1 + j] = bufe[j];
+      rho[b1 + j] = bufr[j] + (k.sigmamed[nr - 1] - md);
+      en[b1 + j] = bufe[j] + (k.energymed[nr - 1] - me);
     }
-    __syncthreads();
-    double mean = 0.0;
-    for (int j = tid; j < ns; j += T) mean += rho[b1 + j];
-    mean = block_sum_dyn(mean, sh) / (double)ns;
-    for (int j = tid; j < ns; j += T) rho[b1 + j] += k.sigmamed[nr - 1] - mean;
-    __syncthreads();
-    mean = 0.0;
-    for (int j = tid; j < ns; j += T) mean += en[b1 + j];
-    mean = block_sum_dyn(mean, sh) / (double)ns;
-    for (int j = tid; j < ns; j += T) en[b1 + j] += k.energymed[nr - 1] - mean;
   }
 }
 

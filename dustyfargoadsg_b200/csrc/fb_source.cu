@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(SRC_MAXW * 32, 2) k_sources(KP k, int ntiles)
     }
   }
   const double ca = SG ? 0.0 : k.cosaz[j], sa = SG ? 0.0 : k.sinaz[j];
-  const double dt = c->dt, om = omf(k);
+  const double dt = c->dt, om = omf(k), domega = k.corot ? c->domega : 0.0;
   // the last substep of a DT leaves the derived fields (fb_download_derived)
   const bool keep = c->done || c->status || c->substeps >= k.cap;
   const bool snap = !SG && c->crash_snap_now;  // the first crash's state (WriteDiskPolar ..., 999)
@@ -167,6 +167,9 @@ __global__ void __launch_bounds__(SRC_MAXW * 32, 2) k_sources(KP k, int ntiles)
     const int t = w * R + q, r = rb + t;
     P[q] = ip[q] = 0.0;
     if (SG || r < 0 || r >= nr) continue;
+    // CorrectVtheta (SideEuler.c:1133-1147): the frame's angular velocity has
+    // just changed by domega (k_planets)
+    if (k.corot) vt[q] -= domega * tab[t][T_RMED];
     P[q] = ENERGY ? (k.gamma - 1.0) * en[q] : rho[q] * tab[t][T_CS] * tab[t][T_CS];
     if (!k.lsa) {
       const double x = tab[t][T_RMED] * ca, y = tab[t][T_RMED] * sa;
