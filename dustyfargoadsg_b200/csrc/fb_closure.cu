@@ -42,7 +42,7 @@
 #define CL_CIN 16    // input feature channels (7 used)
 #define CL_COUT 16   // output channels (2 used: the mass fluxes Fr, Ft)
 #define CL_TILE 64   // pixels per CTA in the convolutions
-#define CL_BS 128
+#define CL_SMS 148
 
 typedef __nv_bfloat16 bf16;
 
@@ -50,16 +50,13 @@ static const int kLayerIn[CL_LAYERS] = {CL_CIN, CL_C, CL_C, CL_C};
 static const int kLayerOut[CL_LAYERS] = {CL_C, CL_C, CL_C, CL_COUT};
 
 // ------------------------------------------------------------ helpers
-static __device__ __forceinline__ float gelu_f(float x)
+// x Phi(x) and, if asked for, its derivative Phi(x) + x phi(x)
+template <bool GRAD>
+static __device__ __forceinline__ float gelu_f(float x, float *grad)
 {
-  return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
-}
-static __device__ __forceinline__ float gelu_grad_f(float x)
-{
-  // d/dx [x Phi(x)] = Phi(x) + x phi(x)
-  const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
-  const float pdf = 0.39894228040143268f * expf(-0.5f * x * x);
-  return cdf + x * pdf;
+  const float e = 1.0f + erff(x * 0.70710678118654752f);
+  if (GRAD) *grad = 0.5f * e + x * (0.39894228040143268f * expf(-0.5f * x * x));
+  return 0.5f * x * e;
 }
 
 static __device__ __forceinline__ unsigned pack_bf16x2(float lo, float hi)
@@ -77,187 +74,277 @@ static __device__ __forceinline__ void mma_bf16(float *d, const unsigned *a, con
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// ------------------------------------------------------------ convolution
-// One CTA: CL_TILE consecutive azimuths of one ring of one sample, all COUT
-// output channels.  4 warps x 16 pixels; per warp COUT/8 n-tiles.
-// MODE 0: hidden layer forward: y = GELU(acc + b) -> bf16, pre-activation -> z (if z)
-// MODE 1: last layer forward: acc + b -> f32
-// MODE 2: backward data: acc * GELU'(zin) -> bf16 (weights transposed/flipped, no bias)
-template <int CIN, int COUT, int MODE>
-__global__ void __launch_bounds__(CL_BS) k_conv(const bf16 *__restrict__ in, const bf16 *__restrict__ w,
-                                                const float *__restrict__ bias, const float *__restrict__ zin,
-                                                bf16 *__restrict__ outb, float *__restrict__ outf,
-                                                float *__restrict__ zout, int nr, int ns)
+// four 8x8 BF16 matrices from shared memory, one row address per lane
+static __device__ __forceinline__ void ldsm4(unsigned *r, const bf16 *p)
 {
-  constexpr int HP = CIN + 8;             // padded pixel stride (elements)
-  constexpr int KW = 9 * CIN + 8;         // padded weight row (elements)
-  __shared__ __align__(16) bf16 halo[3][CL_TILE + 2][HP];
-  __shared__ __align__(16) bf16 wsm[COUT][KW];
-  const int j0 = blockIdx.x * CL_TILE, i = blockIdx.y, b = blockIdx.z;
-  const int tid = threadIdx.x;
-  // input halo: rings i-1..i+1, azimuths j0-1..j0+CL_TILE (periodic), 16-byte chunks
-  constexpr int CH = CIN / 8;  // 16-byte chunks per pixel
-  for (int t = tid; t < 3 * (CL_TILE + 2) * CH; t += CL_BS) {
-    const int c = t % CH, px = (t / CH) % (CL_TILE + 2), r = t / (CH * (CL_TILE + 2));
-    const int ii = i - 1 + r;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+static __device__ __forceinline__ void ldsm4_t(unsigned *r, const bf16 *p)
+{
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((unsigned)__cvta_generic_to_shared(p)));
+}
+static __device__ __forceinline__ void cp16(bf16 *dst, const bf16 *src, bool read)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(read ? 16 : 0));
+}
+static __device__ __forceinline__ void cp8(float2 *dst, const float *src)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+static __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n"); }
+static __device__ __forceinline__ void cp_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+
+// Rows of pixels in shared memory are padded by 8 channels: their stride (48
+// or 80 bytes) puts the eight rows of an ldmatrix in distinct banks.
+#define CL_ROWS 3  // input rows kept: one in use, two on their way
+
+// starts the copy of one ring's azimuths j0-1..j0+CL_TILE (periodic; zeros outside the disc)
+template <int CH, int NTHR>
+static __device__ __forceinline__ void halo_row(bf16 *dst, const bf16 *__restrict__ in, int b, int i, int j0, int nr, int ns)
+{
+  const bool inside = i >= 0 && i < nr;
+  const bf16 *src = inside ? in + ((size_t)b * nr + i) * ns * CH : in;
+  constexpr int Q = CH / 8;  // 16-byte pieces of a pixel
+  for (int t = threadIdx.x; t < (CL_TILE + 2) * Q; t += NTHR) {
+    const int c = t % Q, px = t / Q;
     int jj = j0 - 1 + px;
     jj = jj < 0 ? jj + ns : (jj >= ns ? jj - ns : jj);
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (ii >= 0 && ii < nr) v = *reinterpret_cast<const uint4 *>(in + (((size_t)b * nr + ii) * ns + jj) * CIN + c * 8);
-    *reinterpret_cast<uint4 *>(&halo[r][px][c * 8]) = v;
+    cp16(dst + px * (CH + 8) + c * 8, src + (size_t)(inside ? jj * CH + c * 8 : 0), inside);
   }
-  constexpr int WCH = 9 * CIN / 8;
-  for (int t = tid; t < COUT * WCH; t += CL_BS) {
-    const int c = t % WCH, o = t / WCH;
-    *reinterpret_cast<uint4 *>(&wsm[o][c * 8]) = *reinterpret_cast<const uint4 *>(w + (size_t)o * 9 * CIN + c * 8);
+}
+
+// ------------------------------------------------------------ convolution
+// One CTA: CL_TILE azimuths of `len` consecutive rings of one sample, all COUT
+// output channels; it walks the rings with the input rows in a ring buffer
+// filled two rows ahead.  Each warp takes 16 pixels x 16 output channels and
+// keeps its weights (9*CIN x 16) in registers for the whole walk; a fragment of
+// a row is read once and enters the sums of the three rings that see the row,
+// so a ring costs one barrier and, per six mma, one ldmatrix.  Eight samples of
+// 128x384 cells, against one CTA per 64 pixels that fetched its own weights and
+// read its fragments by single words: 32 -> 32 channels forward 69 -> 50 us
+// (erff and expf of 12.6 M values a layer take most issue slots), back 68 -> 34
+// (the read of g, 4 of 8 bytes a value, started two rings ahead), 32 -> 16
+// channels 38 -> 19, 16 -> 32 forward 41 -> 37.
+// MODE 0: hidden layer forward: y = GELU(acc + b) -> bf16
+// MODE 1: last layer forward: acc + b -> f32
+// MODE 2: backward data: acc * g -> bf16 (weights transposed/flipped, no bias)
+// MODE 3: MODE 0 that also leaves g = GELU'(acc + b) (f32) for the way back,
+//         which then needs neither the pre-activation nor a second erf
+template <int CIN, int COUT, int MODE>
+__global__ void __launch_bounds__(COUT * 8, 512 / (COUT * 8)) k_conv(const bf16 *__restrict__ in, const bf16 *__restrict__ w,
+                                                    const float *__restrict__ bias, const float *__restrict__ gin,
+                                                    bf16 *__restrict__ outb, float *__restrict__ outf,
+                                                    float *__restrict__ gout, int nr, int ns, int len)
+{
+  constexpr int HP = CIN + 8, NTHR = COUT * 8;
+  __shared__ __align__(16) bf16 halo[CL_ROWS][(CL_TILE + 2) * HP];
+  const int j0 = blockIdx.x * CL_TILE, i0 = blockIdx.y * len, i1 = min(i0 + len, nr), b = blockIdx.z;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
+  const int m0 = (warp & 3) * 16, n0 = (warp >> 2) * 16;
+  // g of ring r-1 comes with row r, to a place that only its own thread reads
+  __shared__ float2 gs[MODE == 2 ? CL_ROWS : 1][4][MODE == 2 ? NTHR : 1];
+  auto g_ring = [&](int i) {
+    const float *p = gin + (((size_t)b * nr + i) * ns + j0 + m0 + g) * COUT + n0 + tg * 2;
+#pragma unroll
+    for (int n = 0; n < 2; n++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) cp8(&gs[(i + 1) % CL_ROWS][n * 2 + h][threadIdx.x], p + 8 * h * COUT + n * 8);
+  };
+  for (int r = i0 - 1; r <= i0; r++) {
+    halo_row<CIN, NTHR>(halo[(r + CL_ROWS) % CL_ROWS], in, b, r, j0, nr, ns);
+    cp_commit();
   }
-  __syncthreads();
-  const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, tg = lane & 3;
-  const int m0 = warp * 16;
-  constexpr int NT = COUT / 8;
-  float acc[NT][4];
+  unsigned wr[9 * CIN / 16][2][2];
 #pragma unroll
-  for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+  for (int k = 0; k < 9 * CIN / 16; k++)
 #pragma unroll
-  for (int tap = 0; tap < 9; tap++) {
-    const int dy = tap / 3, dx = tap % 3;  // halo row and column offset (0..2)
-#pragma unroll
-    for (int c0 = 0; c0 < CIN; c0 += 16) {
-      unsigned a[4];
-      a[0] = *reinterpret_cast<const unsigned *>(&halo[dy][m0 + g + dx][c0 + tg * 2]);
-      a[1] = *reinterpret_cast<const unsigned *>(&halo[dy][m0 + g + 8 + dx][c0 + tg * 2]);
-      a[2] = *reinterpret_cast<const unsigned *>(&halo[dy][m0 + g + dx][c0 + 8 + tg * 2]);
-      a[3] = *reinterpret_cast<const unsigned *>(&halo[dy][m0 + g + 8 + dx][c0 + 8 + tg * 2]);
-      const int k0 = tap * CIN + c0;
-#pragma unroll
-      for (int n = 0; n < NT; n++) {
-        unsigned bb[2];
-        bb[0] = *reinterpret_cast<const unsigned *>(&wsm[n * 8 + g][k0 + tg * 2]);
-        bb[1] = *reinterpret_cast<const unsigned *>(&wsm[n * 8 + g][k0 + 8 + tg * 2]);
-        mma_bf16(acc[n], a, bb);
-      }
+    for (int n = 0; n < 2; n++) {
+      const bf16 *p = w + (size_t)(n0 + n * 8 + g) * 9 * CIN + k * 16 + tg * 2;
+      wr[k][n][0] = *reinterpret_cast<const unsigned *>(p);
+      wr[k][n][1] = *reinterpret_cast<const unsigned *>(p + 8);
     }
-  }
-  // epilogue: c0,c1 -> pixel m0+g, c2,c3 -> pixel m0+g+8; channels n*8 + 2tg, +1
+  float2 bv[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+  if (MODE != 2)
 #pragma unroll
-  for (int n = 0; n < NT; n++) {
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int px = m0 + g + 8 * h;
-      const size_t p = ((size_t)b * nr + i) * ns + j0 + px;
-      const int c = n * 8 + tg * 2;
-      float v0 = acc[n][2 * h], v1 = acc[n][2 * h + 1];
-      if (MODE == 0) {
-        v0 += bias[c];
-        v1 += bias[c + 1];
-        if (zout) *reinterpret_cast<float2 *>(zout + p * COUT + c) = make_float2(v0, v1);
-        *reinterpret_cast<unsigned *>(outb + p * COUT + c) = pack_bf16x2(gelu_f(v0), gelu_f(v1));
-      } else if (MODE == 1) {
-        *reinterpret_cast<float2 *>(outf + p * COUT + c) = make_float2(v0 + bias[c], v1 + bias[c + 1]);
-      } else {
-        const float2 z = *reinterpret_cast<const float2 *>(zin + p * COUT + c);
-        *reinterpret_cast<unsigned *>(outb + p * COUT + c) = pack_bf16x2(v0 * gelu_grad_f(z.x), v1 * gelu_grad_f(z.y));
-      }
+    for (int n = 0; n < 2; n++) bv[n] = *reinterpret_cast<const float2 *>(bias + n0 + n * 8 + tg * 2);
+  // this lane's row of the four 8x8 matrices of an A fragment (16 pixels x 16 channels)
+  const int off = (m0 + (lane & 15)) * HP + (lane >> 4) * 8;
+  float acc[3][2][4] = {};  // output rings r-1, r and r+1, as far as the rows up to r go
+  for (int r = i0 - 1; r <= i1; r++) {
+    cp_wait1();
+    __syncthreads();  // row r is here, and row r-1 is no longer read
+    if (r + 2 <= i1) {
+      halo_row<CIN, NTHR>(halo[(r + 2) % CL_ROWS], in, b, r + 2, j0, nr, ns);
+      if (MODE == 2) g_ring(r + 1);
     }
+    cp_commit();
+    const int i = r - 1;  // the ring that row r completes
+    const size_t p0 = ((size_t)b * nr + i) * ns + j0 + m0 + g;
+    const bf16 *row = halo[(r + CL_ROWS) % CL_ROWS] + off;
+#pragma unroll
+    for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+      for (int c0 = 0; c0 < CIN; c0 += 16) {
+        unsigned a[4];
+        ldsm4(a, row + dx * HP + c0);
+#pragma unroll
+        for (int t = 0; t < 3; t++) {  // ring r-1+t sees row r as its row of taps 2-t
+          const int k = (((2 - t) * 3 + dx) * CIN + c0) / 16;
+          mma_bf16(acc[t][0], a, wr[k][0]);
+          mma_bf16(acc[t][1], a, wr[k][1]);
+        }
+      }
+    if (i >= i0) {
+      // c0,c1 -> pixel m0+g, c2,c3 -> pixel m0+g+8; channels n0 + n*8 + 2tg, +1
+#pragma unroll
+      for (int n = 0; n < 2; n++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const size_t q = (p0 + 8 * h) * COUT + n0 + n * 8 + tg * 2;
+          float v0 = acc[0][n][2 * h], v1 = acc[0][n][2 * h + 1];
+          if (MODE == 0 || MODE == 3) {
+            float2 d;
+            v0 = gelu_f<MODE == 3>(v0 + bv[n].x, &d.x);
+            v1 = gelu_f<MODE == 3>(v1 + bv[n].y, &d.y);
+            if (MODE == 3) *reinterpret_cast<float2 *>(gout + q) = d;
+            *reinterpret_cast<unsigned *>(outb + q) = pack_bf16x2(v0, v1);
+          } else if (MODE == 1) {
+            *reinterpret_cast<float2 *>(outf + q) = make_float2(v0 + bv[n].x, v1 + bv[n].y);
+          } else {
+            const float2 d = gs[r % CL_ROWS][n * 2 + h][threadIdx.x];
+            *reinterpret_cast<unsigned *>(outb + q) = pack_bf16x2(v0 * d.x, v1 * d.y);
+          }
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < 2; n++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        acc[0][n][q] = acc[1][n][q];
+        acc[1][n][q] = acc[2][n][q];
+        acc[2][n][q] = 0.f;
+      }
   }
 }
 
 // Weight and bias gradients: gW[o][tap*CIN + c] += sum_p dz[p][o] x[p + off(tap)][c].
-// Each CTA walks `per` tiles (a tile = CL_TILE azimuths of one ring of one
-// sample) accumulating in registers, then adds its partial sums atomically.
-// M = COUT (rows o), N = 9*CIN (columns k), reduction over pixels.
+// M = COUT (rows o), N = 9*CIN (columns k), reduction over pixels.  A CTA walks
+// `len` rings of CL_TILE azimuths as k_conv does.  Both operands lie in shared
+// memory as in global memory, pixel by pixel, and ldmatrix.trans turns them into
+// fragments.  Warps: 3 (one per row of taps) x CL_KW (pixels of a ring); a
+// CTA's sums are added over the CL_KW warps in shared memory and then to gw,
+// four at a time.  Two CTAs of 6 warps on an SM pass their barriers at
+// different times: 32 -> 32 channels, eight samples of 128x384 cells, 250 us
+// with scalar transposes into shared memory, 43 with one CTA of 12 warps, 44
+// with one of 24, 32 with two of 6 and with four of 3 (which add twice the
+// sums to gw).
+#define CL_KW 2
+#define CL_WG_PER_SM 2
+#define CL_WG_ROWS 5  // x rows kept: i-1..i+1 in use, i+2 and i+3 on their way
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(CL_BS) k_conv_wgrad(const bf16 *__restrict__ x, const bf16 *__restrict__ dz,
-                                                      float *__restrict__ gw, float *__restrict__ gb, int nr,
-                                                      int ns, int ntiles, int per)
+__global__ void __launch_bounds__(96 * CL_KW, CL_WG_PER_SM) k_conv_wgrad(const bf16 *__restrict__ x, const bf16 *__restrict__ dz,
+                                                           float *__restrict__ gw, float *__restrict__ gb, int nr,
+                                                           int ns, int len)
 {
-  constexpr int XP = CL_TILE + 2 + 8;  // padded transposed row (pixels)
-  constexpr int DP = CL_TILE + 8;
-  __shared__ __align__(16) bf16 xT[3][CIN][XP];
-  __shared__ __align__(16) bf16 dzT[COUT][DP];
-  constexpr int MT = COUT / 16;           // m16 tiles
-  constexpr int NTT = 9 * CIN / 8;        // n8 tiles in total
-  constexpr int NTW = (NTT + 3) / 4;      // per warp
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tg = lane & 3;
-  float acc[MT][NTW][4];
-#pragma unroll
-  for (int m = 0; m < MT; m++)
-#pragma unroll
-    for (int n = 0; n < NTW; n++) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f;
-  float bsum = 0.f;  // bias gradient of channel tid (tid < COUT)
-  const int tiles_per_ring = ns / CL_TILE;
-  for (int q = 0; q < per; q++) {
-    const int tile = blockIdx.x * per + q;
-    if (tile >= ntiles) break;
-    const int jt = tile % tiles_per_ring, i = (tile / tiles_per_ring) % nr, b = tile / (tiles_per_ring * nr);
-    const int j0 = jt * CL_TILE;
-    __syncthreads();  // previous tile's fragments consumed
-    for (int t = tid; t < 3 * (CL_TILE + 2) * CIN; t += CL_BS) {
-      const int c = t % CIN, px = (t / CIN) % (CL_TILE + 2), r = t / (CIN * (CL_TILE + 2));
-      const int ii = i - 1 + r;
-      int jj = j0 - 1 + px;
-      jj = jj < 0 ? jj + ns : (jj >= ns ? jj - ns : jj);
-      xT[r][c][px] = (ii >= 0 && ii < nr) ? x[(((size_t)b * nr + ii) * ns + jj) * CIN + c] : __float2bfloat16(0.f);
-    }
-    for (int t = tid; t < CL_TILE * COUT; t += CL_BS) {
-      const int o = t % COUT, px = t / COUT;
-      dzT[o][px] = dz[(((size_t)b * nr + i) * ns + j0 + px) * COUT + o];
-    }
+  constexpr int HP = CIN + 8, DP = COUT + 8, NTHR = 96 * CL_KW, DROWS = 3;
+  constexpr int XROW = (CL_TILE + 2) * HP, DROW = CL_TILE * DP;
+  constexpr int MT = COUT / 16, CT = CIN / 16;  // m16 tiles; 16-channel column blocks
+  constexpr int ROWS_B = (CL_WG_ROWS * XROW + DROWS * DROW) * 2, SUM_B = COUT * 9 * CIN * 4;
+  __shared__ __align__(16) unsigned char sm[ROWS_B > SUM_B ? ROWS_B : SUM_B];
+  bf16 *xs = reinterpret_cast<bf16 *>(sm), *ds = xs + CL_WG_ROWS * XROW;
+  const int j0 = blockIdx.x * CL_TILE, i0 = blockIdx.y * len, i1 = min(i0 + len, nr), b = blockIdx.z;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
+  const int dy = warp % 3, kw = warp / 3;
+  auto dz_row = [&](int i) {
+    const bf16 *src = dz + (((size_t)b * nr + i) * ns + j0) * COUT;
+    bf16 *dst = ds + (i % DROWS) * DROW;
+    for (int t = NTHR - 1 - threadIdx.x; t < CL_TILE * COUT / 8; t += NTHR)  // from the end: halo_row starts with warp 0
+      cp16(dst + t / (COUT / 8) * DP + t % (COUT / 8) * 8, src + t * 8, true);
+  };
+  for (int r = -1; r <= 1; r++) halo_row<CIN, NTHR>(xs + (i0 + r + CL_WG_ROWS) % CL_WG_ROWS * XROW, x, b, i0 + r, j0, nr, ns);
+  dz_row(i0);
+  cp_commit();
+  if (i0 + 2 <= i1) halo_row<CIN, NTHR>(xs + (i0 + 2) % CL_WG_ROWS * XROW, x, b, i0 + 2, j0, nr, ns);
+  if (i0 + 1 < i1) dz_row(i0 + 1);
+  cp_commit();
+  float acc[MT][3 * CT * 2][4] = {};
+  float bs[MT][2] = {};  // bias gradient of channels m*16 + g, + 8
+  // this lane's rows (pixels) of the 8x8 matrices of an A and of a B fragment
+  const int aoff = ((lane & 7) + (lane >> 4) * 8) * DP + ((lane >> 3) & 1) * 8;
+  const int boff = (lane & 15) * HP + (lane >> 4) * 8;
+  for (int i = i0; i < i1; i++) {
+    cp_wait1();
     __syncthreads();
-    if (tid < COUT) {
-      float s = 0.f;
-      for (int px = 0; px < CL_TILE; px++) s += __bfloat162float(dzT[tid][px]);
-      bsum += s;
-    }
+    if (i + 3 <= i1) halo_row<CIN, NTHR>(xs + (i + 3) % CL_WG_ROWS * XROW, x, b, i + 3, j0, nr, ns);
+    if (i + 2 < i1) dz_row(i + 2);
+    cp_commit();
+    const bf16 *drow = ds + i % DROWS * DROW + aoff;
+    const bf16 *xrow = xs + (i + dy - 1 + CL_WG_ROWS) % CL_WG_ROWS * XROW + boff;
 #pragma unroll
-    for (int kk = 0; kk < CL_TILE / 16; kk++) {
+    for (int kk = kw * (CL_TILE / CL_KW); kk < (kw + 1) * (CL_TILE / CL_KW); kk += 16) {
       unsigned a[MT][4];
 #pragma unroll
-      for (int m = 0; m < MT; m++) {
-        a[m][0] = *reinterpret_cast<const unsigned *>(&dzT[m * 16 + g][kk * 16 + tg * 2]);
-        a[m][1] = *reinterpret_cast<const unsigned *>(&dzT[m * 16 + g + 8][kk * 16 + tg * 2]);
-        a[m][2] = *reinterpret_cast<const unsigned *>(&dzT[m * 16 + g][kk * 16 + 8 + tg * 2]);
-        a[m][3] = *reinterpret_cast<const unsigned *>(&dzT[m * 16 + g + 8][kk * 16 + 8 + tg * 2]);
-      }
+      for (int m = 0; m < MT; m++) ldsm4_t(a[m], drow + kk * DP + m * 16);
+      if (dy == 0)
 #pragma unroll
-      for (int n = 0; n < NTW; n++) {
-        const int nt = warp * NTW + n;
-        if (nt < NTT) {
-          const int col = nt * 8 + g;            // k = tap*CIN + c
-          const int tap = col / CIN, c = col % CIN;
-          const int dy = tap / 3, dx = tap % 3;
-          const int p0 = kk * 16 + tg * 2 + dx;  // halo column of pixel kk*16 + 2tg
-          const bf16 *row = &xT[dy][c][0];
-          unsigned bb[2];
-          {
-            __nv_bfloat162 v0, v1;
-            v0.x = row[p0]; v0.y = row[p0 + 1];
-            v1.x = row[p0 + 8]; v1.y = row[p0 + 9];
-            bb[0] = *reinterpret_cast<const unsigned *>(&v0);
-            bb[1] = *reinterpret_cast<const unsigned *>(&v1);
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&a[m][q]));
+            bs[m][q & 1] += v.x + v.y;
           }
 #pragma unroll
-          for (int m = 0; m < MT; m++) mma_bf16(acc[m][n], a[m], bb);
+      for (int dx = 0; dx < 3; dx++)
+#pragma unroll
+        for (int c = 0; c < CT; c++) {
+          unsigned bb[4];
+          ldsm4_t(bb, xrow + (kk + dx) * HP + c * 16);
+#pragma unroll
+          for (int m = 0; m < MT; m++) {
+            mma_bf16(acc[m][(dx * CT + c) * 2], a[m], bb);
+            mma_bf16(acc[m][(dx * CT + c) * 2 + 1], a[m], bb + 2);
+          }
         }
-      }
     }
   }
-  // partial sums -> global (rows o = m*16 + g (+8), columns nt*8 + 2tg (+1))
+  float *sum = reinterpret_cast<float *>(sm);
+  for (int t = 0; t < CL_KW; t++) {
+    __syncthreads();
+    if (kw == t)
 #pragma unroll
-  for (int m = 0; m < MT; m++)
+      for (int m = 0; m < MT; m++)
 #pragma unroll
-    for (int n = 0; n < NTW; n++) {
-      const int nt = warp * NTW + n;
-      if (nt < NTT) {
-        const int col = nt * 8 + tg * 2;
-        const int o = m * 16 + g;
-        atomicAdd(gw + (size_t)o * 9 * CIN + col, acc[m][n][0]);
-        atomicAdd(gw + (size_t)o * 9 * CIN + col + 1, acc[m][n][1]);
-        atomicAdd(gw + (size_t)(o + 8) * 9 * CIN + col, acc[m][n][2]);
-        atomicAdd(gw + (size_t)(o + 8) * 9 * CIN + col + 1, acc[m][n][3]);
+        for (int n = 0; n < 3 * CT * 2; n++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            float2 *p = reinterpret_cast<float2 *>(sum + (m * 16 + h * 8 + g) * 9 * CIN + dy * 3 * CIN + n * 8 + tg * 2);
+            float2 v = make_float2(acc[m][n][2 * h], acc[m][n][2 * h + 1]);
+            if (t > 0) {
+              const float2 o = *p;
+              v.x += o.x;
+              v.y += o.y;
+            }
+            *p = v;
+          }
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < COUT * 9 * CIN / 4; t += NTHR)
+    atomicAdd(reinterpret_cast<float4 *>(gw) + t, reinterpret_cast<const float4 *>(sum)[t]);
+  if (dy == 0)
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        float v = bs[m][h];
+        v += __shfl_xor_sync(~0u, v, 1);
+        v += __shfl_xor_sync(~0u, v, 2);
+        if (tg == 0) atomicAdd(gb + m * 16 + h * 8 + g, v);
       }
-    }
-  if (tid < COUT) atomicAdd(gb + tid, bsum);
 }
 
 // ------------------------------------------------------------ features
@@ -557,7 +644,10 @@ struct fb_closure {
   int nr, ns, cap, count;
   cudaStream_t st;
   // per layer: FP32 master weights/biases, BF16 copies, gradients, Adam moments
-  float *w[CL_LAYERS], *b[CL_LAYERS], *gw[CL_LAYERS], *gb[CL_LAYERS];
+  float *w[CL_LAYERS], *b[CL_LAYERS];
+  float *grad;  // gradients of all weights, then of all biases: cleared and read back in one piece
+  float *gw[CL_LAYERS], *gb[CL_LAYERS];
+  int nwt, nbt;  // weights and biases in total
   float *mw[CL_LAYERS], *vw[CL_LAYERS], *mb[CL_LAYERS], *vb[CL_LAYERS];
   bf16 *wf[CL_LAYERS], *wbk[CL_LAYERS];
   int nw[CL_LAYERS];
@@ -577,7 +667,7 @@ struct fb_closure {
   // minibatch work buffers (bmax samples)
   int bmax;
   bf16 *act[CL_LAYERS];   // act[l] = output of layer l (bf16), l < 3
-  float *z[CL_LAYERS];    // pre-activations of layers 0..2
+  float *gp[CL_LAYERS];   // GELU' at the pre-activations of layers 0..2
   float *out;             // last layer output f32
   bf16 *dz[CL_LAYERS];    // gradient w.r.t. each layer's pre-activation
   float *G;               // dL/d(dq)
@@ -655,11 +745,19 @@ extern "C" int fb_closure_create(const fb_ctx *coarse, int capacity, int batch, 
       hw[t] = used ? (float)(sd * cl_gauss(&s)) : 0.0f;
     }
     rc |= cl_alloc((void **)&c->w[l], nw * 4) | cl_alloc((void **)&c->b[l], cout * 4);
-    rc |= cl_alloc((void **)&c->gw[l], nw * 4) | cl_alloc((void **)&c->gb[l], cout * 4);
+    c->nwt += nw;
+    c->nbt += cout;
     rc |= cl_alloc((void **)&c->mw[l], nw * 4) | cl_alloc((void **)&c->vw[l], nw * 4);
     rc |= cl_alloc((void **)&c->mb[l], cout * 4) | cl_alloc((void **)&c->vb[l], cout * 4);
     rc |= cl_alloc((void **)&c->wf[l], nw * 2) | cl_alloc((void **)&c->wbk[l], nw * 2);
     if (!rc) cudaMemcpy(c->w[l], hw.data(), nw * 4, cudaMemcpyHostToDevice);
+  }
+  rc |= cl_alloc((void **)&c->grad, (c->nwt + c->nbt) * 4);
+  c->gw[0] = c->grad;
+  c->gb[0] = c->grad + c->nwt;
+  for (int l = 1; l < CL_LAYERS; l++) {
+    c->gw[l] = c->gw[l - 1] + c->nw[l - 1];
+    c->gb[l] = c->gb[l - 1] + kLayerOut[l - 1];
   }
   rc |= cl_alloc((void **)&c->scale_f, 4 * 4) | cl_alloc((void **)&c->wq_f, 4 * 4);
   rc |= cl_alloc((void **)&c->scale_d, 4 * 8) | cl_alloc((void **)&c->surf_d, c->nr * 8);
@@ -671,7 +769,7 @@ extern "C" int fb_closure_create(const fb_ctx *coarse, int capacity, int batch, 
         cl_alloc((void **)&c->vt_new, n * 8);
   for (int l = 0; l < CL_LAYERS - 1 && !rc; l++) {
     rc |= cl_alloc((void **)&c->act[l], (size_t)batch * n * CL_C * 2);
-    rc |= cl_alloc((void **)&c->z[l], (size_t)batch * n * CL_C * 4);
+    rc |= cl_alloc((void **)&c->gp[l], (size_t)batch * n * CL_C * 4);
   }
   rc |= cl_alloc((void **)&c->out, (size_t)batch * n * CL_COUT * 4);
   for (int l = 0; l < CL_LAYERS && !rc; l++) rc |= cl_alloc((void **)&c->dz[l], (size_t)batch * n * kLayerOut[l] * 2);
@@ -705,11 +803,11 @@ extern "C" int fb_closure_destroy(fb_closure *c)
   if (!c) return FB_OK;
   if (c->st) cudaStreamSynchronize(c->st);
   for (int l = 0; l < CL_LAYERS; l++) {
-    void *p[] = {c->w[l], c->b[l], c->gw[l], c->gb[l], c->mw[l], c->vw[l], c->mb[l], c->vb[l], c->wf[l], c->wbk[l],
-                 c->act[l], c->z[l], c->dz[l]};
+    void *p[] = {c->w[l], c->b[l], c->mw[l], c->vw[l], c->mb[l], c->vb[l], c->wf[l], c->wbk[l],
+                 c->act[l], c->gp[l], c->dz[l]};
     for (void *q : p) cudaFree(q);
   }
-  void *p[] = {c->scale_f, c->wq_f, c->scale_d, c->scale_apply, c->out_sat, c->surf_d, c->surf_f, c->X, c->Y, c->out, c->G,
+  void *p[] = {c->grad, c->scale_f, c->wq_f, c->scale_d, c->scale_apply, c->out_sat, c->surf_d, c->surf_f, c->X, c->Y, c->out, c->G,
                c->loss_part, c->idx, c->stats, c->xin, c->rho_new, c->sig, c->fr, c->ft, c->vt_new};
   for (void *q : p) cudaFree(q);
   if (c->st) cudaStreamDestroy(c->st);
@@ -845,15 +943,44 @@ extern "C" int fb_closure_set_sample(fb_closure *c, int slot, const float *x, co
   return FB_OK;
 }
 
-// forward pass of nb samples whose features start at X (contiguous)
-static void cl_forward(fb_closure *c, const bf16 *X, int nb, int train, cudaStream_t s)
+// Rings a CTA walks: as many CTAs as are resident at once (`per_sm` on each
+// SM), so that the rows shared by two walks and the loads of the weights (or,
+// for their gradients, the sums over the CTAs) are as few as one wave allows.
+static dim3 cl_grid(const fb_closure *c, int nb, int per_sm, int *len)
 {
-  const int nr = c->nr, ns = c->ns;
-  dim3 gr(ns / CL_TILE, nr, nb);
-  k_conv<CL_CIN, CL_C, 0><<<gr, CL_BS, 0, s>>>(X, c->wf[0], c->b[0], NULL, c->act[0], NULL, train ? c->z[0] : NULL, nr, ns);
-  k_conv<CL_C, CL_C, 0><<<gr, CL_BS, 0, s>>>(c->act[0], c->wf[1], c->b[1], NULL, c->act[1], NULL, train ? c->z[1] : NULL, nr, ns);
-  k_conv<CL_C, CL_C, 0><<<gr, CL_BS, 0, s>>>(c->act[1], c->wf[2], c->b[2], NULL, c->act[2], NULL, train ? c->z[2] : NULL, nr, ns);
-  k_conv<CL_C, CL_COUT, 1><<<gr, CL_BS, 0, s>>>(c->act[2], c->wf[3], c->b[3], NULL, NULL, c->out, NULL, nr, ns);
+  const int units = c->ns / CL_TILE * nb;
+  int walks = CL_SMS * per_sm / units;
+  walks = walks < 1 ? 1 : (walks > c->nr ? c->nr : walks);
+  *len = (c->nr + walks - 1) / walks;
+  return dim3(c->ns / CL_TILE, (c->nr + *len - 1) / *len, nb);
+}
+
+template <int CIN, int COUT, int MODE>
+static void cl_conv(const fb_closure *c, const bf16 *in, const bf16 *w, const float *bias, const float *gin, bf16 *outb,
+                    float *outf, float *gout, int nb, cudaStream_t s)
+{
+  int len;
+  const dim3 gr = cl_grid(c, nb, 512 / (COUT * 8), &len);
+  k_conv<CIN, COUT, MODE><<<gr, COUT * 8, 0, s>>>(in, w, bias, gin, outb, outf, gout, c->nr, c->ns, len);
+}
+
+template <int CIN, int COUT>
+static void cl_wgrad(const fb_closure *c, const bf16 *x, int l, int nb, cudaStream_t s)
+{
+  int len;
+  const dim3 gr = cl_grid(c, nb, CL_WG_PER_SM, &len);
+  k_conv_wgrad<CIN, COUT><<<gr, 96 * CL_KW, 0, s>>>(x, c->dz[l], c->gw[l], c->gb[l], c->nr, c->ns, len);
+}
+
+// forward pass of nb samples whose features start at X (contiguous); HIDDEN
+// is the hidden layers' mode: 3 when the way back follows, 0 otherwise
+template <int HIDDEN>
+static void cl_layers(fb_closure *c, const bf16 *X, int nb, cudaStream_t s)
+{
+  cl_conv<CL_CIN, CL_C, HIDDEN>(c, X, c->wf[0], c->b[0], NULL, c->act[0], NULL, c->gp[0], nb, s);
+  cl_conv<CL_C, CL_C, HIDDEN>(c, c->act[0], c->wf[1], c->b[1], NULL, c->act[1], NULL, c->gp[1], nb, s);
+  cl_conv<CL_C, CL_C, HIDDEN>(c, c->act[1], c->wf[2], c->b[2], NULL, c->act[2], NULL, c->gp[2], nb, s);
+  cl_conv<CL_C, CL_COUT, 1>(c, c->act[2], c->wf[3], c->b[3], NULL, NULL, c->out, NULL, nb, s);
 }
 
 // loss and gradients of the samples idx[0..nb) (gathered into the batch)
@@ -876,28 +1003,21 @@ static int cl_loss_grad(fb_closure *c, const int *hidx, int nb, double *loss)
                       cudaMemcpyDeviceToDevice, s);
   }
   cudaMemcpyAsync(c->idx, hidx, nb * 4, cudaMemcpyHostToDevice, s);
-  cl_forward(c, xb, nb, 1, s);
+  cl_layers<3>(c, xb, nb, s);
   const int nblk = (int)((n * nb + 255) / 256);
   k_loss<<<nblk, 256, 0, s>>>(c->out, c->Y, c->sig, c->idx, c->scale_f, c->wq_f, c->surf_f, c->G, c->loss_part, nr, ns,
                               nb);
   k_loss_adjoint<<<nblk, 256, 0, s>>>(c->G, c->sig, c->idx, c->scale_f, c->surf_f, c->dz[3], nr, ns, nb);
-  dim3 gr(ns / CL_TILE, nr, nb);
-  // backward data: dz[l-1] = conv^T(dz[l]) * GELU'(z[l-1])
-  k_conv<CL_COUT, CL_C, 2><<<gr, CL_BS, 0, s>>>(c->dz[3], c->wbk[3], NULL, c->z[2], c->dz[2], NULL, NULL, nr, ns);
-  k_conv<CL_C, CL_C, 2><<<gr, CL_BS, 0, s>>>(c->dz[2], c->wbk[2], NULL, c->z[1], c->dz[1], NULL, NULL, nr, ns);
-  k_conv<CL_C, CL_C, 2><<<gr, CL_BS, 0, s>>>(c->dz[1], c->wbk[1], NULL, c->z[0], c->dz[0], NULL, NULL, nr, ns);
+  // backward data: dz[l-1] = conv^T(dz[l]) * GELU'(pre-activation of l-1)
+  cl_conv<CL_COUT, CL_C, 2>(c, c->dz[3], c->wbk[3], NULL, c->gp[2], c->dz[2], NULL, NULL, nb, s);
+  cl_conv<CL_C, CL_C, 2>(c, c->dz[2], c->wbk[2], NULL, c->gp[1], c->dz[1], NULL, NULL, nb, s);
+  cl_conv<CL_C, CL_C, 2>(c, c->dz[1], c->wbk[1], NULL, c->gp[0], c->dz[0], NULL, NULL, nb, s);
   // weight gradients
-  for (int l = 0; l < CL_LAYERS; l++) {
-    cudaMemsetAsync(c->gw[l], 0, c->nw[l] * 4, s);
-    cudaMemsetAsync(c->gb[l], 0, kLayerOut[l] * 4, s);
-  }
-  const int ntiles = nb * nr * (ns / CL_TILE);
-  const int per = (ntiles + 148 * 4 - 1) / (148 * 4);
-  const int nbw = (ntiles + per - 1) / per;
-  k_conv_wgrad<CL_CIN, CL_C><<<nbw, CL_BS, 0, s>>>(xb, c->dz[0], c->gw[0], c->gb[0], nr, ns, ntiles, per);
-  k_conv_wgrad<CL_C, CL_C><<<nbw, CL_BS, 0, s>>>(c->act[0], c->dz[1], c->gw[1], c->gb[1], nr, ns, ntiles, per);
-  k_conv_wgrad<CL_C, CL_C><<<nbw, CL_BS, 0, s>>>(c->act[1], c->dz[2], c->gw[2], c->gb[2], nr, ns, ntiles, per);
-  k_conv_wgrad<CL_C, CL_COUT><<<nbw, CL_BS, 0, s>>>(c->act[2], c->dz[3], c->gw[3], c->gb[3], nr, ns, ntiles, per);
+  cudaMemsetAsync(c->grad, 0, (c->nwt + c->nbt) * 4, s);
+  cl_wgrad<CL_CIN, CL_C>(c, xb, 0, nb, s);
+  cl_wgrad<CL_C, CL_C>(c, c->act[0], 1, nb, s);
+  cl_wgrad<CL_C, CL_C>(c, c->act[1], 2, nb, s);
+  cl_wgrad<CL_C, CL_COUT>(c, c->act[2], 3, nb, s);
   if (!contiguous) cudaFreeAsync(xb, s);
   if (loss) {
     std::vector<double> lp(nblk);
@@ -919,13 +1039,8 @@ extern "C" int fb_closure_loss_grad(fb_closure *c, int first, int nb, double *lo
   for (int q = 0; q < nb; q++) idx[q] = first + q;
   int rc = cl_loss_grad(c, idx.data(), nb, loss);
   if (rc) return rc;
-  size_t ow = 0, ob = 0;
-  for (int l = 0; l < CL_LAYERS; l++) {
-    if (gw && cudaMemcpy(gw + ow, c->gw[l], c->nw[l] * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return FB_ERR_CUDA;
-    if (gb && cudaMemcpy(gb + ob, c->gb[l], kLayerOut[l] * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return FB_ERR_CUDA;
-    ow += c->nw[l];
-    ob += kLayerOut[l];
-  }
+  if (gw && cudaMemcpy(gw, c->grad, c->nwt * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return FB_ERR_CUDA;
+  if (gb && cudaMemcpy(gb, c->grad + c->nwt, c->nbt * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return FB_ERR_CUDA;
   return FB_OK;
 }
 
@@ -976,7 +1091,7 @@ extern "C" int fb_closure_infer(fb_closure *c, const fb_ctx *coarse, int slot, f
     if (cudaStreamSynchronize(cs) != cudaSuccess) return FB_ERR_CUDA;
     x = c->xin;
   }
-  cl_forward(c, x, 1, 0, s);
+  cl_layers<0>(c, x, 1, s);
   if (cudaMemcpyAsync(out, c->out, n * CL_COUT * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)
     return FB_ERR_CUDA;
@@ -994,11 +1109,7 @@ extern "C" int fb_closure_apply(fb_closure *c, fb_ctx *coarse)
   cl_features(c, coarse, c->xin, s);
   // the network on the disc's stream (weights are only written by training)
   const int nr = c->nr, ns = c->ns;
-  dim3 gr(ns / CL_TILE, nr, 1);
-  k_conv<CL_CIN, CL_C, 0><<<gr, CL_BS, 0, s>>>(c->xin, c->wf[0], c->b[0], NULL, c->act[0], NULL, NULL, nr, ns);
-  k_conv<CL_C, CL_C, 0><<<gr, CL_BS, 0, s>>>(c->act[0], c->wf[1], c->b[1], NULL, c->act[1], NULL, NULL, nr, ns);
-  k_conv<CL_C, CL_C, 0><<<gr, CL_BS, 0, s>>>(c->act[1], c->wf[2], c->b[2], NULL, c->act[2], NULL, NULL, nr, ns);
-  k_conv<CL_C, CL_COUT, 1><<<gr, CL_BS, 0, s>>>(c->act[2], c->wf[3], c->b[3], NULL, NULL, c->out, NULL, nr, ns);
+  cl_layers<0>(c, c->xin, 1, s);
   k_saturate<<<256, 256, 0, s>>>(c->out, c->out_sat, (size_t)nr * ns * CL_COUT);
   k_face_flux<<<dim3((ns + 127) / 128, nr + 1), 128, 0, s>>>(*kp, c->out_sat, (double)c->h_scale[0] * c->gain, c->fr,
                                                                c->ft);
