@@ -355,10 +355,8 @@ extern "C" int fb_create(const fb_params *p, const double *radii, fb_ctx **out)
   k.cs_ring = dtable(ctx, cs_ring.data(), nr);
   k.gcs = dalloc(ctx, nr);
   k.p15 = dtable(ctx, p15.data(), nr);
-  k.dxrad = dtable(ctx, dxrad.data(), nr);
   k.dxtheta = dtable(ctx, dxth.data(), nr);
   k.invdxtheta = dtable(ctx, invdxth.data(), nr);
-  k.dxtheta_cfl = dtable(ctx, dxth_cfl.data(), nr);
   k.mindx2 = dtable(ctx, mindx2.data(), nr);
   k.supp_torque = dalloc(ctx, nr);
   k.sigmamed = dalloc(ctx, nr);

@@ -109,8 +109,7 @@ struct KP {
   const double *cs_ring;   // isothermal sound speed per ring
   double *gcs;             // GLOBAL_SoundSpeed (ring means of cs)
   const double *p15;       // pow(Rmed, 1.5)
-  const double *dxrad, *dxtheta, *invdxtheta, *mindx2;
-  const double *dxtheta_cfl; // Rmed*(PMAX-PMIN)/ns as ConditionCFL forms it (SourceEuler.c:1344)
+  const double *dxtheta, *invdxtheta, *mindx2;
   const double *supp_torque;
   const double *sigmamed, *energymed, *vthetamed, *vradmed;
   const double *betatab;   // ComputeBetaCooling(Rmed)
@@ -397,7 +396,6 @@ void fb_launch_edges(const KP &k, cudaStream_t s);  // open / non-reflecting edg
 // constant = SETCONSTANTOPACITY; conv = 0.1 unit_length^-2 unit_mass
 void fb_launch_opacity(const KP &k, int constant, double imposed, double factor, double unit_temperature,
                        double unit_mass, double inv_l3, double conv, cudaStream_t s);
-void fb_launch_floors_boundary(const KP &k, cudaStream_t s);
 void fb_launch_damping(const KP &k, double dt_override, cudaStream_t s);
 void fb_launch_vr_damping(const KP &k, cudaStream_t s);  // both in one launch (discs with walls)
 // the end of a substep in one pass (discs with walls, small grids): vr, floors,

@@ -25,9 +25,9 @@
 // scratch and must be serialised by the caller.
 #include <cuda_runtime.h>
 #include <math.h>
-#include <pthread.h>
 #include <stdio.h>
 #include <string.h>
+#include <mutex>
 #include "fb_dev.cuh"
 
 #define FB_NA_MAX_CELLS 131072   // (nrad+1)*nsec limit, = FB_NOALLOC_MAX_CELLS
@@ -47,13 +47,12 @@ struct na_device {
   double *tables;
   fb_ctl *ctl;
   int smem_ns[2];    // largest nsec the azimuthal kernel attributes were set for
-  cudaEvent_t copied;
+  std::mutex lock;   // held while htab is filled and until its copy is done
+  double htab[FB_NA_NTAB * (FB_NA_MAX_NRAD + 1)];
 };
 
 static na_device g_na[FB_NA_MAX_DEVICES];
-static pthread_mutex_t g_na_lock = PTHREAD_MUTEX_INITIALIZER;
-static double g_na_htab[FB_NA_NTAB * (FB_NA_MAX_NRAD + 1)];
-static cudaEvent_t g_na_busy;  // recorded behind the last copy from g_na_htab (NULL: none yet)
+static std::mutex g_na_setup;
 static __thread char g_na_err[256];
 
 extern "C" const char *fb_noalloc_last_error(void) { return g_na_err; }
@@ -79,10 +78,6 @@ static int na_setup(int dev)
       cudaGetSymbolAddress((void **)&d.ctl, fb_na_ctl) != cudaSuccess) {
     cudaGetLastError();
     return na_fail(FB_ERR_CUDA, "cudaGetSymbolAddress failed for the no-alloc scratch");
-  }
-  if (!d.copied && cudaEventCreateWithFlags(&d.copied, cudaEventDisableTiming) != cudaSuccess) {
-    cudaGetLastError();
-    return na_fail(FB_ERR_CUDA, "an event could not be created");
   }
   // the azimuthal variants (all of them, whatever the grid) and the radial
   // and vr passes
@@ -116,27 +111,27 @@ extern "C" int fb_transport_noalloc(const fb_params *p, double *dens, double *vr
   const cudaError_t ce = cudaStreamIsCapturing(s, &cap);
   if (ce != cudaSuccess || cap != cudaStreamCaptureStatusNone)
     return na_fail(FB_ERR_CUDA, ce != cudaSuccess ? cudaGetErrorString(ce) : "the stream is capturing a graph");
-  pthread_mutex_lock(&g_na_lock);
-  int rc = na_setup(dev);
   na_device &d = g_na[dev];
+  std::unique_lock<std::mutex> hold(d.lock);
+  int rc;
+  {
+    std::lock_guard<std::mutex> one(g_na_setup);
+    rc = na_setup(dev);
+  }
   const int ei = p->energy_equation ? 1 : 0;
   if (rc == FB_OK && d.smem_ns[ei] < ns) {
     rc = fb_gas_prepare(ns, p->energy_equation);
     if (rc == FB_OK) d.smem_ns[ei] = ns;
     else na_fail(rc, "shared-memory attributes for the azimuthal pass could not be set");
   }
-  if (rc != FB_OK) {
-    pthread_mutex_unlock(&g_na_lock);
-    return rc;
-  }
+  if (rc != FB_OK) return rc;
   // 1-D geometry of FillPolar1DArrays (src/SourceEuler.c:80-123) into a
   // static host table, then into the static device table.
   const int T = nr + 1;
-  double *rinf = g_na_htab, *rsup = rinf + T, *rmed = rsup + T, *surf = rmed + T;
+  double *rinf = d.htab, *rsup = rinf + T, *rmed = rsup + T, *surf = rmed + T;
   double *invrmed = surf + T, *invsurf = invrmed + T, *invdiffrmed = invsurf + T;
   double *dxth = invdiffrmed + T, *invdxth = dxth + T, *radii = invdxth + T;
-  if (g_na_busy) cudaEventSynchronize(g_na_busy);
-  memset(g_na_htab, 0, sizeof(double) * FB_NA_NTAB * T);
+  memset(d.htab, 0, sizeof(double) * FB_NA_NTAB * T);
   {
     const double drrsep = (p->rmax - p->rmin) / (double)nr, span = log(p->rmax / p->rmin);
     for (int i = 0; i <= nr; i++)
@@ -156,20 +151,18 @@ extern "C" int fb_transport_noalloc(const fb_params *p, double *dens, double *vr
     rinf[nr] = radii[nr];
     for (int i = 1; i < nr; i++) invdiffrmed[i] = 1.0 / (rmed[i] - rmed[i - 1]);
   }
-  cudaError_t e = cudaMemcpyAsync(d.tables, g_na_htab, sizeof(double) * FB_NA_NTAB * T,
+  cudaError_t e = cudaMemcpyAsync(d.tables, d.htab, sizeof(double) * FB_NA_NTAB * T,
                                   cudaMemcpyHostToDevice, s);
   // the outflow accumulator is the only scratch value read before written
   if (e == cudaSuccess) e = cudaMemsetAsync(&d.ctl->lost_mass, 0, sizeof(double), s);
   // A call that returns its outflow waits for the stream at its end, so it need
-  // not wait here too: the next call does, before it writes to the host table
-  // (128x384 cells: 66 -> 59 us a call).
-  if (e == cudaSuccess) e = cudaEventRecord(d.copied, s);
-  if (e == cudaSuccess) g_na_busy = d.copied;
+  // not wait for the copy here too; it keeps the lock until then (128x384
+  // cells: 66 -> 59 us a call).
   if (e != cudaSuccess || !lost_mass) {
     const cudaError_t w = cudaStreamSynchronize(s);
     if (e == cudaSuccess) e = w;
+    hold.unlock();
   }
-  pthread_mutex_unlock(&g_na_lock);
   if (e != cudaSuccess) return na_fail(FB_ERR_CUDA, cudaGetErrorString(e));
 
   KP k;
@@ -207,11 +200,11 @@ extern "C" int fb_transport_noalloc(const fb_params *p, double *dens, double *vr
   k.transport_only = 1;
   fb_launch_transport(k, dt, s);
   e = cudaGetLastError();
-  if (e != cudaSuccess) return na_fail(FB_ERR_CUDA, cudaGetErrorString(e));
   if (lost_mass) {
-    e = cudaMemcpyAsync(lost_mass, &d.ctl->lost_mass, sizeof(double), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return na_fail(FB_ERR_CUDA, cudaGetErrorString(e));
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(lost_mass, &d.ctl->lost_mass, sizeof(double), cudaMemcpyDeviceToHost, s);
+    const cudaError_t w = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = w;
   }
-  return FB_OK;
+  return e == cudaSuccess ? FB_OK : na_fail(FB_ERR_CUDA, cudaGetErrorString(e));
 }

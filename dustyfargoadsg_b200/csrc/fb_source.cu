@@ -18,6 +18,14 @@
 // neighbouring ring's from the thread's own registers or, across warps,
 // through a row in shared memory, one barrier per step.  So every field is
 // read once and only the final velocities and energy are written.
+//
+// What bounds it: FP64 issue and the latency of each step's chain (divisions,
+// roots); the five kernels it replaces, one cell a thread, spent their time on
+// 4-5 passes over memory and on launches.  Isothermal 768x2304: 126 us in
+// launches of their own -> 70 (280.6 -> 246.7 a substep), 333x1001 with energy
+// 116.9 -> 107.9 a substep, 128x384 51.5 -> 47.3, 48x144 45.3 -> 41.9.  A
+// version that marched down a column lost on small grids (48x144: 54 a
+// substep): a ring's chain of some 4,800 cycles is then serial.
 #define SRC_MAXW 16  // warps per CTA
 #define SRC_LEFT 3
 #define SRC_CO 27    // 32 - SRC_LEFT - 2
