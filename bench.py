@@ -60,6 +60,7 @@ STAGE_BYTES = {
     "substep1": (64, 64), "source_terms": (40, 56), "substep3": (0, 40),
     "transport_radial": (64, 80), "transport_azimuthal": (80, 96),
     "transport_vr_boundary": (40, 40), "transport_ring_means": (8, 8),
+    "finish": (48, 72),
 }
 
 
