@@ -3521,11 +3521,13 @@ __global__ void __launch_bounds__(MT, 2) k_finish(KP k, int fuse_cs, cudaGraphCo
     double *pp = k.partials + (size_t)i * 5;  // summed by the controller in ring order
     for (int q = 0; q < 5; q++) pp[q] = s[1 + q];
   }
-  const int flags = __syncthreads_or(negd | (nege << 1) | (bad << 2));
-  if (tid == 0) {
-    if (flags & 1) atomicOr(&k.ctl->neg_dens_flag, 1);
-    if (flags & 2) atomicOr(&k.ctl->neg_energy_flag, 1);
-    if (flags & 4) atomicOr(&k.ctl->nonfinite, 1);
+  // DetectCrash, as in k_cfl.  (The barrier's OR is a predicate's, so three
+  // conditions need three of them; a warp's is bitwise.)
+  const unsigned flags = __reduce_or_sync(0xffffffffu, (unsigned)(negd | (nege << 1) | (bad << 2)));
+  if (flags && (tid & 31) == 0) {
+    if (flags & 1u) atomicOr(&k.ctl->neg_dens_flag, 1);
+    if (flags & 2u) atomicOr(&k.ctl->neg_energy_flag, 1);
+    if (flags & 4u) atomicOr(&k.ctl->nonfinite, 1);
   }
   if (i >= 1) {
     const double viscosity = nu_ring(k, i);
