@@ -108,18 +108,21 @@ __global__ void __launch_bounds__(SRC_MAXW * 32, 2) k_sources(KP k, int ntiles)
   int j = (tile * SRC_CO + m) % ns;
   if (j < 0) j += ns;
   // every global load first
-  double rho[R], en[R], vr[R], vt[R], pot[R], ar[R], at[R];
+  double rho[R], en[R], vr[R], vt[R], pot[R], ip[R], ar[R], at[R];
 #pragma unroll
   for (int q = 0; q < R; q++) {
     const int r = rb + w * R + q;
-    rho[q] = en[q] = vr[q] = vt[q] = pot[q] = ar[q] = at[q] = 0.0;
+    rho[q] = en[q] = vr[q] = vt[q] = pot[q] = ip[q] = ar[q] = at[q] = 0.0;
     if (r >= 0 && r < nr) {
       const size_t l = (size_t)r * ns + j;
       rho[q] = k.rho[l];
       if (ENERGY) en[q] = k.e[l];
       vr[q] = SG ? k.vri[l] : k.vr[l];
       vt[q] = SG ? k.vti[l] : k.vt[l];
-      if (!SG && k.lsa) pot[q] = k.pot[l];
+      if (!SG && k.lsa) {  // k_potential has left both
+        pot[q] = k.pot[l];
+        if (PART) ip[q] = k.indpot[l];
+      }
       if (SG) {
         ar[q] = k.sg_accr[l];
         at[q] = k.sg_acct[l];
@@ -169,11 +172,11 @@ __global__ void __launch_bounds__(SRC_MAXW * 32, 2) k_sources(KP k, int ntiles)
   __syncthreads();
   // ---- pressure and potential
   const bool use_ind = (!k.discard_gas_it) && (fabs(k.pmax - k.pmin - 2. * M_PI) < 0.01);
-  double P[R], ip[R];
+  double P[R];
 #pragma unroll
   for (int q = 0; q < R; q++) {
     const int t = w * R + q, r = rb + t;
-    P[q] = ip[q] = 0.0;
+    P[q] = 0.0;
     if (SG || r < 0 || r >= nr) continue;
     // CorrectVtheta (SideEuler.c:1133-1147): the frame's angular velocity has
     // just changed by domega (k_planets)
@@ -206,7 +209,7 @@ __global__ void __launch_bounds__(SRC_MAXW * 32, 2) k_sources(KP k, int ntiles)
         k.pres[l] = P[q];
         if (!k.lsa) k.pot[l] = pot[q];
       }
-      if (PART) k.indpot[l] = ip[q];  // IndPotential (Pframeforce.c:55-121)
+      if (PART && !k.lsa) k.indpot[l] = ip[q];  // IndPotential (Pframeforce.c:55-121)
       if (snap) {
         k.crash_snap[l] = rho[q];
         k.crash_snap[ncell + l] = vr[q];
