@@ -793,8 +793,9 @@ static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NU
     // applies its change before the gas update (SourceEuler.c:476-525)
     if (k.lsa) STAGE(ST_POT, 2, fb_launch_lsa_modes(k, s));
     STAGE(ST_CFL, 1, fb_launch_planets(k, NULL, s));
-    // (k_sources applies the change of the frame where it runs from the state)
-    if (k.self_gravity) STAGE(ST_CFL, 1, fb_launch_correct_vtheta(k, s));
+    // (k_sources applies the change of the frame where it runs from the state
+    // and no particles read it before)
+    if (k.self_gravity || ctx->has_dust) STAGE(ST_CFL, 1, fb_launch_correct_vtheta(k, s));
     cudaEventRecord(ctx->ev_planets, s);
   } else {
     // the planets' step on a branch of its own: no gas kernel of the substep
@@ -813,8 +814,10 @@ static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NU
   // the particles read (the state, and the half of the gradient grids the
   // previous substep wrote), so the particles run beside them; with the energy
   // equation the sound speed they read changes before that, and the
-  // self-gravity kicks write the grids they read: in line there.
-  const bool dust_branch = ctx->has_dust && !ctx->profiling && !k.energy && !k.self_gravity;
+  // self-gravity kicks write the grids they read: in line there.  In line too
+  // with a corotating frame, which has no fork point behind the limits (the
+  // planets' step runs in line).
+  const bool dust_branch = ctx->has_dust && !ctx->profiling && !k.energy && !k.self_gravity && !k.corot;
   if (dust_branch) {
     cudaStreamWaitEvent(ctx->st_dust, ctx->ev_fork, 0);
     fb_launch_dust_substep(k, ctx->pp, ctx->st_dust, ctx->st_rng, ctx->ev_fork, ctx->ev_dust_rng, ctx->ev_planets,

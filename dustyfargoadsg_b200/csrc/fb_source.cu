@@ -179,8 +179,9 @@ __global__ void __launch_bounds__(SRC_MAXW * 32, 2) k_sources(KP k, int ntiles)
     P[q] = 0.0;
     if (SG || r < 0 || r >= nr) continue;
     // CorrectVtheta (SideEuler.c:1133-1147): the frame's angular velocity has
-    // just changed by domega (k_planets)
-    if (k.corot) vt[q] -= domega * tab[t][T_RMED];
+    // just changed by domega (k_planets).  Particles have read the corrected
+    // state before this pass: k_correct_vtheta ran then.
+    if (!PART && k.corot) vt[q] -= domega * tab[t][T_RMED];
     P[q] = ENERGY ? (k.gamma - 1.0) * en[q] : rho[q] * tab[t][T_CS] * tab[t][T_CS];
     if (!k.lsa) {
       const double x = tab[t][T_RMED] * ca, y = tab[t][T_RMED] * sa;
