@@ -275,16 +275,19 @@ static __device__ __forceinline__ long long candidate_limit(const PP &pp, int np
   return lim < pp.ncand ? lim : pp.ncand;
 }
 
-// The acceptance of every candidate a substep can need: it depends on the
-// stream's position alone, so it runs beside the drift and the ranking that
-// find how many are needed.
-__global__ void __launch_bounds__(D_BS) k_rng_count(PP pp)
+// The candidates' acceptance.  It depends on the stream's position alone, so
+// where the particles have streams of their own (ahead = 1) it runs beside the
+// drift and the ranking that find how many candidates are needed, for all that
+// a substep can need; in line it runs behind them, for those alone.
+__global__ void __launch_bounds__(D_BS) k_rng_count(PP pp, int ahead)
 {
   fb_grid_dependency();
   __shared__ int sh[D_BS / 32];
   const long long c = (long long)blockIdx.x * D_BS + threadIdx.x;
+  const int npairs = ahead ? 0 : pp.dc->npairs;
+  const long long need = ahead ? pp.ncand : npairs > 0 ? candidate_limit(pp, npairs) : 0;
   int acc = 0;
-  if (c < pp.ncand) {
+  if (c < need) {
     double u1, u2, w;
     acc = candidate(pp.dc->x, c, &u1, &u2, &w) ? 1 : 0;
   }
@@ -301,8 +304,8 @@ __global__ void __launch_bounds__(D_BS) k_rng_count(PP pp)
 
 // Accepted candidate number g (in stream order) becomes pair g.  The
 // blocks' counts are summed here: each block that holds a needed candidate adds
-// the counts before it; block 0 also checks that the candidates cover the pairs needed -- never silently
-// wrong: the step stops with an error status.
+// the counts before it; block 0 also checks that the candidates cover the
+// pairs needed -- never silently wrong: the step stops with an error status.
 __global__ void __launch_bounds__(D_BS) k_rng_scatter(KP k, PP pp, int nb)
 {
   fb_grid_dependency();
@@ -749,7 +752,7 @@ void fb_launch_dust_substep(const KP &k, const PP &pp, cudaStream_t s, cudaStrea
   const int ncb = (pp.ncand + D_BS - 1) / D_BS;
   if (pp.feel_turb && srng != s) {
     cudaStreamWaitEvent(srng, fork, 0);
-    fb_launch(k_rng_count, ncb, D_BS, 0, srng, pp);
+    fb_launch(k_rng_count, ncb, D_BS, 0, srng, pp, 1);
     cudaEventRecord(rng_done, srng);
   }
   fb_launch(k_dust_drift, nb, D_BS, 0, s, k, pp);
@@ -760,7 +763,7 @@ void fb_launch_dust_substep(const KP &k, const PP &pp, cudaStream_t s, cudaStrea
     if (srng != s)
       cudaStreamWaitEvent(s, rng_done, 0);
     else
-      fb_launch(k_rng_count, ncb, D_BS, 0, s, pp);
+      fb_launch(k_rng_count, ncb, D_BS, 0, s, pp, 0);
     fb_launch(k_rng_scatter, ncb, D_BS, 0, s, k, pp, ncb);
   }
   if (planets_done) cudaStreamWaitEvent(s, planets_done, 0);  // positions after the planets' step
