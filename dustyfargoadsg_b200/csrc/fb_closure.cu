@@ -1051,9 +1051,12 @@ extern "C" int fb_closure_loss_grad(fb_closure *c, int first, int nb, double *lo
   for (int q = 0; q < nb; q++) idx[q] = first + q;
   int rc = cl_loss_grad(c, idx.data(), nb, loss);
   if (rc) return rc;
-  if (gw && cudaMemcpy(gw, c->grad, c->nwt * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return FB_ERR_CUDA;
-  if (gb && cudaMemcpy(gb, c->grad + c->nwt, c->nbt * 4, cudaMemcpyDeviceToHost) != cudaSuccess) return FB_ERR_CUDA;
-  return FB_OK;
+  // on the network's own stream, for which no other waits (without a loss
+  // cl_loss_grad has not waited either)
+  if (gw && cudaMemcpyAsync(gw, c->grad, c->nwt * 4, cudaMemcpyDeviceToHost, c->st) != cudaSuccess) return FB_ERR_CUDA;
+  if (gb && cudaMemcpyAsync(gb, c->grad + c->nwt, c->nbt * 4, cudaMemcpyDeviceToHost, c->st) != cudaSuccess)
+    return FB_ERR_CUDA;
+  return cudaStreamSynchronize(c->st) == cudaSuccess ? FB_OK : FB_ERR_CUDA;
 }
 
 // `iters` Adam steps on random minibatches of `nb` samples drawn from

@@ -63,3 +63,35 @@ def test_loss_and_gradients(tmp_path, nr, ns, batch):
         for got, ref, at, size in ((gw, rw, ow, n), (gb, rb, ob, cout)):
             assert np.linalg.norm((got - ref)[at:at + size]) <= 1e-2 * np.linalg.norm(ref[at:at + size])
         ow, ob = ow + n, ob + cout
+
+
+def test_gradients_without_a_loss(tmp_path):
+    """The loss is optional: without it the gradients are the same ones.
+    Tolerance: two runs add the CTAs' FP32 sums in another order, at most some
+    300 partial sums of 6e-8 each; 1e-5 of the norm."""
+    from dustyfargoadsg_b200 import Disc, _ffi, read_par
+    nr, ns, batch = 96, 256, 8
+    params = R.init_params(seed=3, scale=0.6)
+    rng = np.random.RandomState(1)
+    with Disc(read_par(_oracle.write_par(ISO, str(tmp_path), Nrad=nr, Nsec=ns))) as disc:
+        lib = disc.lib
+        c = _closure(disc, batch, batch)
+        try:
+            wt, bt = R.flatten(params)
+            _ffi.check(lib.fb_closure_params(c, _fp(wt), _fp(bt), 0), "params")
+            _ffi.check(lib.fb_closure_scales(c, _dp(np.array([0.02, 1.0, 1.0])), _dp(np.array([1.5, 1.0, 1.0])), 0),
+                       "scales")
+            for s in range(batch):
+                x, y = rng.uniform(-1, 1, (nr, ns, 16)), rng.standard_normal((3, nr, ns)) * 0.05
+                _ffi.check(lib.fb_closure_set_sample(c, s, _fp(x.astype(np.float32)), _fp(y.astype(np.float32)),
+                                                     _fp(np.ones(nr, dtype=np.float32))), "sample")
+            runs = []
+            for loss in (C.byref(C.c_double()), None, None, None):
+                gw, gb = np.zeros_like(wt), np.zeros_like(bt)
+                _ffi.check(lib.fb_closure_loss_grad(c, 0, batch, loss, _fp(gw), _fp(gb)), "loss_grad")
+                runs.append((gw, gb))
+        finally:
+            lib.fb_closure_destroy(c)
+    for got in runs[1:]:
+        for g, w in zip(got, runs[0]):
+            assert np.linalg.norm(w) > 0.0 and np.linalg.norm(g - w) <= 1e-5 * np.linalg.norm(w)
