@@ -754,6 +754,11 @@ static bool cs_at_end(const fb_ctx *ctx)
   const KP &k = ctx->k;
   return cfl_at_end(k) && k.energy && !ctx->has_dust && !k.ent_diff && !k.rad_diff;
 }
+// walls: vr and the damping in one launch, where any ring damps
+static bool vr_with_damping(const KP &k)
+{
+  return !cfl_at_end(k) && !edges_other_than_wall(k) && k.evanescent && k.n_damp_rings > 0;
+}
 static bool more_substeps(const fb_ctx *ctx) { return cfl_at_end(ctx->k) ? ctx->h_ctl->go : !ctx->h_ctl->done; }
 
 static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NULL)
@@ -876,8 +881,7 @@ static int enqueue_substep(fb_ctx *ctx, const cudaGraphConditionalHandle *h = NU
     if (fb_azi_launches(kt) == 2) STAGE(ST_TVMED, 1, fb_launch_azi_vmed(kt, 0.0, s));
     STAGE(ST_TAZI, 1, fb_launch_transport_azimuthal(kt, 0.0, s, true));
   }
-  // walls: vr and the damping in one launch, where any ring damps
-  const bool vr_damp = !at_end && !edges_other_than_wall(k) && k.evanescent && k.n_damp_rings > 0;
+  const bool vr_damp = vr_with_damping(k);
   if (vr_damp)
     STAGE(ST_TVR, 1, fb_launch_vr_damping(k, s));
   else if (!at_end)
@@ -1703,18 +1707,24 @@ extern "C" int fb_tune(fb_ctx *ctx, int substeps, fb_tuning *best, double *ms_ou
   Snapshot sn;
   rc = snapshot_take(ctx, sn);
   if (rc) { snapshot_free(sn); fb_profile(ctx, 0); return rc; }
-  const int cell_stages[] = {ST_POT, ST_SUB1, ST_SUB3, ST_TVR};
+  // the stages of this disc that launch k.cell_bs threads a CTA; without any
+  // the width stays as it is
+  int cell_stages[4], ncell = 0;
+  if (k.lsa || k.self_gravity) cell_stages[ncell++] = ST_POT;
+  if (k.self_gravity) cell_stages[ncell++] = ST_SUB1;
+  if (k.energy) cell_stages[ncell++] = ST_SUB3;
+  if (!cfl_at_end(k) && !vr_with_damping(k)) cell_stages[ncell++] = ST_TVR;
   const int azi_stage[] = {ST_TAZI};
   const int rad_stage[] = {ST_TRAD};
   double total = 0.0;
   // 1. per-cell CTA width
-  {
+  if (ncell > 0) {
     const int cand[] = {64, 128, 256};
     int bestv = k.cell_bs;
     double bestms = 1e300;
     for (int c : cand) {
       k.cell_bs = c;
-      const double ms = tune_measure(ctx, sn, substeps, cell_stages, 4);
+      const double ms = tune_measure(ctx, sn, substeps, cell_stages, ncell);
       if (ms >= 0.0 && ms < bestms) { bestms = ms; bestv = c; }
     }
     k.cell_bs = bestv;

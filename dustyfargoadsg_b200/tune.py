@@ -6,7 +6,9 @@ each grid size of the batched sweep and keeps a table of the fastest,
                          "rad_columns": .., "rad_rings": .., "ms_per_substep": ..}, ...},
      "energy": {...}}
 
-which Disc(..., tuning=table) and the batch apply per grid.  Each timed disc
+which Disc(..., tuning=table) and the batch apply per grid (ms_per_substep is
+the time of the tuned stages, not of the substep; cell_block is kept where no
+stage of the disc has it).  Each timed disc
 is also recorded in a manifest line (its parameters, the shapes tried and
 the result) so that the sweep's runs can be reused as training inputs.
 

@@ -98,3 +98,18 @@ def test_tile_variant_on_short_rings(tmp_path, E):
     for v in (6, 7, 8):
         for k in FIELDS + ("energy",):
             np.testing.assert_array_equal(out[1][k], out[v][k], err_msg="%s variant %d" % (k, v))
+
+
+@pytest.mark.parametrize("nr,ns,tuned", [(48, 144, False), (300, 40, False), (48, 144, True)])
+def test_width_is_tuned_where_a_stage_has_it(tmp_path, nr, ns, tuned):
+    """An isothermal disc with walls launches no kernel of cell_block threads (its
+    substep ends in k_finish, or beyond 296 rings in k_vr_damping), so the tuner
+    leaves the width as it was set; open edges bring one that has it."""
+    from dustyfargoadsg_b200 import Disc, read_par, tune
+    over = dict(wall_boundary=0, open_inner=1) if tuned else {}
+    p = read_par(os.path.join(_oracle.CONFIG_DIR, "iso_128x384.par"), nrad=nr, nsec=ns, **over)
+    with Disc(p, noise=1e-4, seed=0) as d:
+        d.set_tuning({"cell_block": 192})
+        entry = tune.tune_disc(d, substeps=2)
+    assert (entry["cell_block"] in (64, 128, 256)) if tuned else (entry["cell_block"] == 192)
+    assert 0.0 < entry["ms_per_substep"] < 10.0
