@@ -83,3 +83,70 @@ def test_transport_noalloc_refuses_oversized_grid(tmp_path):
     rc = lib.fb_transport_noalloc(C.byref(p), dummy, dummy, dummy, dummy, 0.01, None, None)
     assert rc == -1
     assert b"too large" in lib.fb_noalloc_last_error()
+
+
+def _call(lib, p, t, dt, stream=None, lost=None):
+    ptr = [C.c_void_p(t[q].data_ptr()) for q in range(4)]
+    return lib.fb_transport_noalloc(C.byref(p), *ptr, dt, C.c_void_p(stream),
+                                    C.byref(lost) if lost is not None else None)
+
+
+def test_calls_in_a_row_reuse_the_host_table(tmp_path):
+    """Back-to-back calls on one stream, grids and calls with and without
+    lost_mass alternating: a call must not see the tables of the next one, and
+    each gives what a call on its own gives, to the last bit."""
+    import torch
+
+    import dustyfargoadsg_b200 as fb
+    lib = fb.load()
+    adi = os.path.join(_oracle.CONFIG_DIR, "adiabatic_sg_512x1536.par")
+    runs = []
+    for nr, ns, dt in ((48, 144, 0.02), (130, 390, 0.004), (17, 61, 0.03)):
+        p = fb.read_par(adi, nrad=nr, nsec=ns, self_gravity=0)
+        with fb.Disc(p, noise=1e-2, seed=nr) as disc:
+            s = disc.download()
+        start = torch.tensor(np.stack([s[k] for k in FIELDS]), device="cuda")
+        alone, lost = start.clone(), C.c_double()
+        torch.cuda.synchronize()
+        assert _call(lib, p, alone, dt, lost=lost) == 0
+        torch.cuda.synchronize()
+        runs.append((p, dt, start, alone, lost.value))
+    outs = []
+    work = [(n, bool(with_lost), runs[n][2].clone()) for n, with_lost in
+            ((0, 0), (1, 0), (2, 1), (1, 1), (0, 0), (2, 0), (0, 1), (1, 0), (2, 0))]
+    torch.cuda.synchronize()
+    for n, with_lost, t in work:
+        lost = C.c_double() if with_lost else None
+        assert _call(lib, runs[n][0], t, runs[n][1], lost=lost) == 0
+        outs.append(lost.value if with_lost else None)
+    torch.cuda.synchronize()
+    for (n, _, t), lost in zip(work, outs):
+        assert torch.equal(t, runs[n][3])
+        assert lost is None or lost == runs[n][4]
+
+
+def test_call_on_a_capturing_stream_is_refused(tmp_path):
+    """With an error, leaving the capture valid; the next call works."""
+    import torch
+
+    import dustyfargoadsg_b200 as fb
+    lib = fb.load()
+    p = fb.read_par(os.path.join(_oracle.CONFIG_DIR, "iso_128x384.par"), nrad=32, nsec=96)
+    with fb.Disc(p, noise=1e-4, seed=1) as disc:
+        s = disc.download()
+    start = torch.tensor(np.stack([s[k] for k in FIELDS]), device="cuda")
+    t, x, lost = start.clone(), torch.zeros(8, device="cuda"), C.c_double()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    for given in (lost, None):
+        with torch.cuda.graph(graph, stream=stream):
+            x.add_(1.0)
+            rc = _call(lib, p, t, 0.01, stream=stream.cuda_stream, lost=given)
+        assert rc == -3 and b"capturing" in lib.fb_noalloc_last_error()  # FB_ERR_CUDA
+        graph.replay()
+        torch.cuda.synchronize()
+        graph.reset()
+    assert float(x.sum()) == 16.0 and torch.equal(t, start)
+    assert _call(lib, p, t, 0.01, lost=lost) == 0
+    torch.cuda.synchronize()
+    assert not torch.equal(t, start) and bool(torch.isfinite(t).all())
