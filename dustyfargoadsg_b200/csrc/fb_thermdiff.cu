@@ -532,10 +532,11 @@ static cudaLaunchConfig_t sorc_config(const KP &k, int C, cudaLaunchAttribute *a
 
 // CTAs of the cluster that solves this grid, 0 where the grid-wide kernel
 // does: the largest cluster the device schedules, 16 (which functions must opt
-// into) or 8, that holds the grid.
+// into) or 8, that holds the grid.  Its colours' planes need an even nsec; a
+// parameter file with an odd one is refused, overrides of its fields are not.
 static int sorc_size(const KP &k)
 {
-  if (k.nr < 4) return 0;
+  if (k.nr < 4 || (k.ns & 1)) return 0;
   const void *fns[SORC_M] = {(const void *)k_sor_cluster<1>, (const void *)k_sor_cluster<2>,
                              (const void *)k_sor_cluster<3>};
   for (int C = SORC_MAX; C >= 8; C /= 2) {

@@ -58,7 +58,8 @@ CASES = {
     "dust_adi": (ADI, 13, 40, 2, dict(BOULDERS, self_gravity=0)),
     "dust_sg_adi": (ADI, 16, 48, 2, dict(BOULDERS, dust_feel_sg=1)),
     "dust_sg_iso": (DUST, 16, 48, 1, dict(BOULDERS, self_gravity=1, sgthicknesssmoothing=0.3, dust_feel_sg=1)),
-    # pairs that a parameter file cannot ask for; overrides can
+    # what a parameter file cannot ask for; overrides can
+    "adi_implicit_odd": (ADI, 13, 41, 1, dict(self_gravity=0, radiative_diffusion=2)),
     "dust_lsa": (DUST, 13, 40, 2, dict(BOULDERS, **LSA)),
     "dust_corot": (DUST, 13, 40, 2, dict(BOULDERS, corotating=1)),
 }
