@@ -477,18 +477,24 @@ static __device__ double dev_aspect_ratio(const KP &k, double rad)
   return aspectratio;
 }
 
-// DerivMotionRK5 (RungeKunta.c:13-53)
-static __device__ void rk5_deriv(const double *q, const double *masses, double *deriv, int n,
+// DerivMotionRK5 (RungeKunta.c:13-53).  One thread runs each instruction a few
+// times, so what it costs is fetching them: one copy of the code for the six
+// stages and no unrolled loops (two free planets: k_planets 52 us parity, 57
+// fast with six copies, 27 and 26 so; with FeelOthers 61 and 66, 32 and 31).
+static __device__ __noinline__ void rk5_deriv(const double *q, const double *masses, double *deriv, int n,
                                  double dt, const int *feelothers, int indirect, double *Dist)
 {
   const double *x = q, *y = q + n, *vx = q + 2 * n, *vy = q + 3 * n;
   double *dx = deriv, *dy = deriv + n, *dvx = deriv + 2 * n, *dvy = deriv + 3 * n;
+#pragma unroll 1
   for (int i = 0; i < n; i++) Dist[i] = sqrt(x[i] * x[i] + y[i] * y[i]);
+#pragma unroll 1
   for (int i = 0; i < n; i++) {
     dx[i] = vx[i];
     dy[i] = vy[i];
     dvx[i] = -FB_G * 1.0 / Dist[i] / Dist[i] / Dist[i] * x[i];
     dvy[i] = -FB_G * 1.0 / Dist[i] / Dist[i] / Dist[i] * y[i];
+#pragma unroll 1
     for (int j = 0; j < n; j++) {
       if (indirect) {
         dvx[i] -= FB_G * masses[j] / Dist[j] / Dist[j] / Dist[j] * x[j];
@@ -502,6 +508,7 @@ static __device__ void rk5_deriv(const double *q, const double *masses, double *
       }
     }
   }
+#pragma unroll 1
   for (int i = 0; i < 4 * n; i++) deriv[i] *= dt;
 }
 
@@ -509,28 +516,31 @@ static __device__ void rk5_deriv(const double *q, const double *masses, double *
 static __device__ void rk5(const double *q0, double dt, const double *masses, double *q1, int n,
                            const int *feelothers, int indirect, RkWork &w)
 {
-  // k2..k5 enter the first translations multiplied by 0.0; the reference
-  // seeds them with the previous call's k6 (RungeKunta.c:73-75), which is
-  // finite, so zeros give the same sums.
+  // the reference adds the later stages too, multiplied by 0.0
+  // (RungeKunta.c:73-91): finite values, which leave the sums as they are
   double *k1 = w.k[0], *k2 = w.k[1], *k3 = w.k[2], *k4 = w.k[3], *k5 = w.k[4], *k6 = w.k[5];
   double *Dist = w.dist;
   const int m = 4 * n;
-  for (int s = 0; s < 6; s++)
-    for (int i = 0; i < m; i++) w.k[s][i] = 0.0;
   rk5_deriv(q0, masses, k1, n, dt, feelothers, indirect, Dist);
-  for (int i = 0; i < m; i++) q1[i] = q0[i] + 0.2 * k1[i] + 0.0 * k2[i] + 0.0 * k3[i] + 0.0 * k4[i] + 0.0 * k5[i];
+#pragma unroll 1
+  for (int i = 0; i < m; i++) q1[i] = q0[i] + 0.2 * k1[i];
   rk5_deriv(q1, masses, k2, n, dt, feelothers, indirect, Dist);
-  for (int i = 0; i < m; i++) q1[i] = q0[i] + 0.075 * k1[i] + 0.225 * k2[i] + 0.0 * k3[i] + 0.0 * k4[i] + 0.0 * k5[i];
+#pragma unroll 1
+  for (int i = 0; i < m; i++) q1[i] = q0[i] + 0.075 * k1[i] + 0.225 * k2[i];
   rk5_deriv(q1, masses, k3, n, dt, feelothers, indirect, Dist);
-  for (int i = 0; i < m; i++) q1[i] = q0[i] + 0.3 * k1[i] + -0.9 * k2[i] + 1.2 * k3[i] + 0.0 * k4[i] + 0.0 * k5[i];
+#pragma unroll 1
+  for (int i = 0; i < m; i++) q1[i] = q0[i] + 0.3 * k1[i] + -0.9 * k2[i] + 1.2 * k3[i];
   rk5_deriv(q1, masses, k4, n, dt, feelothers, indirect, Dist);
+#pragma unroll 1
   for (int i = 0; i < m; i++)
-    q1[i] = q0[i] + -11.0 / 54.0 * k1[i] + 2.5 * k2[i] + -70.0 / 27.0 * k3[i] + 35.0 / 27.0 * k4[i] + 0.0 * k5[i];
+    q1[i] = q0[i] + -11.0 / 54.0 * k1[i] + 2.5 * k2[i] + -70.0 / 27.0 * k3[i] + 35.0 / 27.0 * k4[i];
   rk5_deriv(q1, masses, k5, n, dt, feelothers, indirect, Dist);
+#pragma unroll 1
   for (int i = 0; i < m; i++)
     q1[i] = q0[i] + 1631.0 / 55296.0 * k1[i] + 175.0 / 512.0 * k2[i] + 575.0 / 13824.0 * k3[i] +
             44275.0 / 110592.0 * k4[i] + 253.0 / 4096.0 * k5[i];
   rk5_deriv(q1, masses, k6, n, dt, feelothers, indirect, Dist);
+#pragma unroll 1
   for (int i = 0; i < m; i++)
     q1[i] = q0[i] + 37.0 / 378.0 * k1[i] + 250.0 / 621.0 * k3[i] + 125.0 / 594.0 * k4[i] + 512.0 / 1771.0 * k6[i];
 }
