@@ -54,10 +54,11 @@ CONFIG_DIR = os.path.join(REPO, "dustyfargoadsg_b200", "configs")
 FALLBACK_HBM_GBS = 6650.0
 
 # Algorithmic bytes per cell of each stage (distinct fields read + written,
-# 8 B each), isothermal / with energy equation.
+# 8 B each), isothermal / with energy equation; "_sg": with self-gravity, where
+# the stage also reads the two accelerations.
 STAGE_BYTES = {
     "cfl_forces": (32, 40), "potential": (8, 8), "soundspeed": (0, 24),
-    "substep1": (64, 64), "source_terms": (40, 56), "substep3": (0, 40),
+    "substep1": (64, 64), "source_terms": (40, 56), "source_terms_sg": (56, 72), "substep3": (0, 40),
     "transport_radial": (64, 80), "transport_azimuthal": (80, 96),
     "transport_vr_boundary": (40, 40), "transport_ring_means": (8, 8),
     "finish": (48, 72),
@@ -383,7 +384,8 @@ def main():
             best = name
     roofline = None
     if best is not None:
-        bpc = STAGE_BYTES.get(best, (None, None))[energy]
+        sg = best + "_sg" if p.self_gravity else best
+        bpc = STAGE_BYTES.get(sg, STAGE_BYTES.get(best, (None, None)))[energy]
         ms, cnt = prof[best]
         if nsub > 0:
             cnt = nsub  # the time of one pass of the stage

@@ -41,7 +41,7 @@
 #define CL_C 32      // hidden channels
 #define CL_CIN 16    // input feature channels (7 used)
 #define CL_COUT 16   // output channels (2 used: the mass fluxes Fr, Ft)
-#define CL_TILE 64   // pixels per CTA in the convolutions
+#define CL_TILE 64   // azimuths of the rings that a CTA of the convolutions walks
 #define CL_SMS 148
 
 typedef __nv_bfloat16 bf16;

@@ -74,8 +74,8 @@ struct fb_lsa {
   double s[FB_LSA_MAX_MODES], cp[FB_LSA_MAX_MODES], sp[FB_LSA_MAX_MODES];
 };
 
-#define FB_LIM_TAB 10  // doubles per ring of KP::lim_tab
-#define FB_SRC_TAB 14  // doubles per ring of KP::src_tab
+#define FB_LIM_TAB 10  // doubles per ring of KP::lim_tab (nine, padded to pairs)
+#define FB_SRC_TAB 12  // doubles per ring of KP::src_tab
 
 // Everything a kernel needs, passed by value (well under the 32 KB limit).
 struct KP {

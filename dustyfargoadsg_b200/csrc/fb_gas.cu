@@ -1005,7 +1005,7 @@ static __device__ __forceinline__ double vischeat_of(const KP &k, int i, double 
 // alone without it), ComputeViscousHeating (SourceEuler.c:1554-1606) and
 // SubStep3 (SourceEuler.c:1119-1302; pdV, viscous heating, beta cooling) in
 // one pass: a cell's stresses feed its own heating, so they are evaluated
-// here (and still stored) instead of read back.  Ring 0's heating is
+// here and never stored.  Ring 0's heating is
 // extrapolated from rings 1 and 2, whose stresses its threads evaluate too.
 // Reads the velocities and the energy that k_sources left and writes Energy =
 // EnergyNew (ring nr stays zero).  DivV and the heating are stored by the last

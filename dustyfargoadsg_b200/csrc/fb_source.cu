@@ -31,9 +31,10 @@
 #define SRC_CO 27    // 32 - SRC_LEFT - 2
 #define SRC_HALO 5   // rows of the CTA's tile that are halo: three below, two above
 
-// per-ring table rows (fb_source_table)
+// per-ring table rows: fb_source_table's, then those that each CTA fills in
 enum { T_RINF, T_RSUP, T_RMED, T_INVRMED, T_INVDIFFRMED, T_INVDIFFRSUP, T_INVRINF, T_INVDXTHETA, T_C0, T_C1, T_P15,
-       T_CS, T_TORQUE, T_NU, T_N = FB_SRC_TAB };
+       T_CS, T_TORQUE, T_NU, T_N };
+static_assert(T_TORQUE == FB_SRC_TAB, "the rows of fb_source_table");
 
 int fb_source_tiles(int ns) { return (ns + SRC_CO - 1) / SRC_CO; }
 
@@ -41,7 +42,7 @@ void fb_source_table(const fb_geom *g, const double *invdxtheta, const double *p
 {
   const int nr = g->nr;
   for (int i = 0; i < nr; i++) {
-    double *t = out + (size_t)i * T_N;
+    double *t = out + (size_t)i * FB_SRC_TAB;
     t[T_RINF] = g->rinf[i];
     t[T_RSUP] = g->rsup[i];
     t[T_RMED] = g->rmed[i];
@@ -154,9 +155,9 @@ __global__ void __launch_bounds__(SRC_MAXW * 32, 2) k_sources(KP k, int ntiles)
     for (int t = threadIdx.x; t < nw * R; t += blockDim.x) {
       const int r = rb + t;
       if (r < 0 || r >= nr) continue;
-      const double *g = k.src_tab + (size_t)r * T_N;
+      const double *g = k.src_tab + (size_t)r * FB_SRC_TAB;
 #pragma unroll
-      for (int f = 0; f < T_TORQUE; f++) tab[t][f] = g[f];
+      for (int f = 0; f < FB_SRC_TAB; f++) tab[t][f] = g[f];
       tab[t][T_TORQUE] = k.supp_torque[r];
       // FViscosity(Rmed[r]) (Viscosity.c:23-69)
       tab[t][T_NU] = (k.visc_mode == 1) ? k.alpha * k.gcs[r] * k.gcs[r] * g[T_P15] : k.nu_const;

@@ -343,7 +343,8 @@ int fb_planet_force(fb_ctx *ctx, double x, double y, double rsmoothing, double m
    fb_get_tuning reports the values in effect.  fb_tune times the candidates
    on the context's own disc, `substeps` substeps each from a saved state
    that it restores (the disc does not advance), keeps the fastest and
-   reports the summed ms per substep of the tuned stages. */
+   reports the summed ms per substep of the tuned stages.  The CTA width is
+   left alone where the disc's substep launches no kernel of that width. */
 typedef struct fb_tuning {
   int cell_block, azi_cells_per_thread, rad_columns, rad_rings;
   int azi_variant;  /* 0 automatic, 1 narrow (NQ+3 shared rings), 2 wide (2 NQ+1 rings),
