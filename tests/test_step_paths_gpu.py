@@ -98,3 +98,43 @@ def test_step_path_matches_recording(name, mode):
         scale = np.hypot(want["pl_x"], want["pl_y"]) if k in ("pl_x", "pl_y") else np.abs(w)
         err = np.max(np.abs(g - w)) / (np.max(scale) or 1.0)
         assert err <= (TOL_DUST if k.startswith("pc_") else TOL_GAS), (k, err)
+
+
+@pytest.mark.parametrize("par", [ISO, ADI])
+def test_damping_towards_the_initial_profiles(par):
+    """The stage that the recorded discs' substeps end with, against numpy:
+    EvanescentBoundary (src/SideEuler.c:796-950) with DampToIni and ZeroVradBC.
+    Bar of the stages: 1e-12 of each field's largest value."""
+    import dustyfargoadsg_b200 as fb
+    from dustyfargoadsg_b200._ffi import FB_STAGE_DAMPING
+    nr, ns, dt = 24, 72, 0.03
+    p = fb.read_par(os.path.join(fb.CONFIG_DIR, par), nrad=nr, nsec=ns, self_gravity=0, rmin=0.4, rmax=2.5, wkzrmin=0.5,
+                    wkzrmax=2.1, **INI)
+    with fb.Disc(p, noise=1e-2, seed=4) as d:
+        d.step()
+        prof = {k: d.prof[k].copy() for k in ("sigma_med", "vtheta_med", "vrad_med", "energy_med")}
+        f = {k: v.reshape(nr + 1, ns) for k, v in d.download().items() if k in GAS}
+        d.stage(FB_STAGE_DAMPING, dt)
+        got = d.download()
+    radii = p.rmin * np.exp(np.arange(nr + 1) / nr * np.log(p.rmax / p.rmin))
+    rmed = 2.0 / 3.0 * np.diff(radii ** 3) / np.diff(radii ** 2)
+    zeroed = damped = 0
+    for i in range(nr):
+        lo, hi = rmed[i] < p.wkzrmin, rmed[i] > p.wkzrmax
+        if not (lo or hi):
+            continue
+        damped += 1
+        ref, end = (p.wkzrmin, rmed[0]) if lo else (p.wkzrmax, rmed[-1])
+        lam = ((rmed[i] - ref) / (end - ref)) ** 2 * dt / (p.dampingtodynamicaltimeratio * rmed[i] ** 1.5)
+        target = dict(dens=prof["sigma_med"][i], vtheta=prof["vtheta_med"][i], vrad=prof["vrad_med"][i],
+                      energy=prof["energy_med"][i])
+        zero = (lo and i <= 1) or (hi and i == nr - 1)
+        zeroed += zero
+        for k in GAS[:3] + ((GAS[3],) if p.energy_equation else ()):
+            f[k][i] = (f[k][i] + lam * target[k]) / (1.0 + lam)
+            if zero and k != "energy":
+                f[k][i] = 0.0 if k == "vrad" else target[k]
+    assert zeroed >= 2 and damped > zeroed
+    for k in GAS:
+        err = np.max(np.abs(got[k] - f[k].ravel())) / (np.max(np.abs(f[k])) or 1.0)
+        assert err <= 1e-12, (k, err)
