@@ -316,7 +316,10 @@ int fb_download_crash(fb_ctx *ctx, fb_state *st, double *crash_time);
 /* Derived output fields at the current state (reference layout, (nrad+1)*nsec):
    which = 0 Temperature (src/SourceEuler.c:2440), 1 Potential, 2 Pressure,
    3 SoundSpeed, 4 DivergenceVelocity, 5 ViscHeat, 6 SG radial acceleration
-   (SG_Accr, src/sgacc.c:152-161), 7 SG azimuthal acceleration (SG_Acct). */
+   (SG_Accr, src/sgacc.c:152-161), 7 SG azimuthal acceleration (SG_Acct).
+   1, 2, 4 and 5 are what the last substep of the last DT left; a DT that an
+   error stopped behind a substep's source terms (an edge that is not
+   reproduced, too few candidate pairs) may leave the DT before's. */
 int fb_download_derived(fb_ctx *ctx, int which, double *out);
 /* Rings [ring0, ring0+nrings) of the self-gravity accelerations last
    computed (by the step, or by fb_stage(.., FB_STAGE_SELFGRAV, ..)): SG_Accr
